@@ -124,7 +124,7 @@ GG_DEV void dp45_vjp(const DevParams& P, const double x[4], const double v[4], d
 #pragma unroll
       for (int i = 0; i < 4; ++i) k[s][i] = kst[s][i];
     } else {
-      Geometry<kMetricKerr> G;
+      Geometry<kMetricKerr, kStepperDP45> G;
       G.at(P, px[1], px[2]);
       G.accel(w, k[s]);
     }
