@@ -405,35 +405,25 @@ GG_DEV double fifth_root(double x) {
 // 50.8 ms (full Dormand-Prince); a 256^2 Schwarzschild render 2.28 / 2.09 ms.
 constexpr double kSteadyErr = 0.5625;
 
-// Dormand-Prince tableau (geodesic.rs:210-242).
-struct DP {
-  static constexpr double a2 = 1.0 / 5.0, a3 = 3.0 / 10.0, a4 = 4.0 / 5.0, a5 = 8.0 / 9.0;
-  static constexpr double b21 = 1.0 / 5.0;
-  static constexpr double b31 = 3.0 / 40.0, b32 = 9.0 / 40.0;
-  static constexpr double b41 = 44.0 / 45.0, b42 = -56.0 / 15.0, b43 = 32.0 / 9.0;
-  static constexpr double b51 = 19372.0 / 6561.0, b52 = -25360.0 / 2187.0,
-                          b53 = 64448.0 / 6561.0, b54 = -212.0 / 729.0;
-  static constexpr double b61 = 9017.0 / 3168.0, b62 = -355.0 / 33.0, b63 = 46732.0 / 5247.0,
-                          b64 = 49.0 / 176.0, b65 = -5103.0 / 18656.0;
-  static constexpr double c1 = 35.0 / 384.0, c3 = 500.0 / 1113.0, c4 = 125.0 / 192.0,
-                          c5 = -2187.0 / 6784.0, c6 = 11.0 / 84.0;
-  static constexpr double d1 = 5179.0 / 57600.0, d3 = 7571.0 / 16695.0, d4 = 393.0 / 640.0,
-                          d5 = -92097.0 / 339200.0, d6 = 187.0 / 2100.0, d7 = 1.0 / 40.0;
+// Dormand-Prince tableau (geodesic.rs:210-242), in constant memory: a 64-bit
+// immediate would take two moves at every use.
+struct RefTable {
+  double a[6];     // stage nodes; a[0] = 0
+  double b[6][5];  // stage velocity weights
+  double c[6];     // 5th-order weights, c[1] = 0
+  double d[7];     // 4th-order weights, d[1] = 0
 };
-
-// Stage position pos + (h a_i) vel (the reference moves stage positions
-// along the step's initial velocity, geodesic.rs:248-284); returns false
-// when the reference's is_valid_position would reject it.
-// Uncontracted like the reference's `pos + h*a*vel`, so the last stage's
-// position (ha = h) equals the accepted position bit for bit, which is what
-// lets k7 serve as the next step's k1.
-GG_DEV bool stage_pos(const Ray& R, double ha, double& r, double& th) {
-  const double t = add_rn(R.x[0], mul_rn(ha, R.v[0]));
-  r = add_rn(R.x[1], mul_rn(ha, R.v[1]));
-  th = add_rn(R.x[2], mul_rn(ha, R.v[2]));
-  const double ph = add_rn(R.x[3], mul_rn(ha, R.v[3]));
-  return finite4(t, r, th, ph) && r > 0.0;
-}
+__constant__ RefTable kRef = {
+    {0.0, 1.0 / 5.0, 3.0 / 10.0, 4.0 / 5.0, 8.0 / 9.0, 1.0},
+    {{0.0},
+     {1.0 / 5.0},
+     {3.0 / 40.0, 9.0 / 40.0},
+     {44.0 / 45.0, -56.0 / 15.0, 32.0 / 9.0},
+     {19372.0 / 6561.0, -25360.0 / 2187.0, 64448.0 / 6561.0, -212.0 / 729.0},
+     {9017.0 / 3168.0, -355.0 / 33.0, 46732.0 / 5247.0, 49.0 / 176.0, -5103.0 / 18656.0}},
+    {35.0 / 384.0, 0.0, 500.0 / 1113.0, 125.0 / 192.0, -2187.0 / 6784.0, 11.0 / 84.0},
+    {5179.0 / 57600.0, 0.0, 7571.0 / 16695.0, 393.0 / 640.0, -92097.0 / 339200.0, 187.0 / 2100.0,
+     1.0 / 40.0}};
 
 // Where the stage derivatives k1..k6 live between the stages of an attempt
 // (and k1 between attempts): this thread's column of a block-shared array,
@@ -441,36 +431,84 @@ GG_DEV bool stage_pos(const Ray& R, double ha, double& r, double& th) {
 // out of registers, they free 48 registers of the stepping loop for
 // occupancy.
 struct KStore {
-  double (*s)[4][kTraceBlock];  // [7][4][kTraceBlock], declared by the kernel
-  GG_DEV double& operator()(int stage, int i) const { return s[stage][i][threadIdx.x]; }
+  double2 (*s)[2][kTraceBlock];  // [7][2][kTraceBlock], declared by the kernel
+  GG_DEV double operator()(int stage, int i) const {
+    return reinterpret_cast<const double*>(&s[stage][i >> 1][threadIdx.x])[i & 1];
+  }
+  GG_DEV void get(int stage, double k[4]) const {
+    const double2 a = s[stage][0][threadIdx.x], b = s[stage][1][threadIdx.x];
+    k[0] = a.x;
+    k[1] = a.y;
+    k[2] = b.x;
+    k[3] = b.y;
+  }
+  GG_DEV void set(int stage, const double k[4]) const {
+    s[stage][0][threadIdx.x] = make_double2(k[0], k[1]);
+    s[stage][1][threadIdx.x] = make_double2(k[2], k[3]);
+  }
 };
 
 // The same store in a per-thread array (local memory).
 struct KStoreLocal {
   double (*k)[4];  // [7][4]
-  GG_DEV double& operator()(int stage, int i) const { return k[stage][i]; }
+  GG_DEV double operator()(int stage, int i) const { return k[stage][i]; }
+  GG_DEV void get(int stage, double out[4]) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[i] = k[stage][i];
+  }
+  GG_DEV void set(int stage, const double in[4]) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) k[stage][i] = in[i];
+  }
 };
 
 // v + h (c1 k1 + c3 k3 + c4 k4 + c5 k5 + c6 k6), left to right, uncontracted
 // (geodesic.rs:294-295).
 GG_DEV double combine5(double v, double h, double k1, double k3, double k4, double k5,
                        double k6) {
-  double s = add_rn(mul_rn(DP::c1, k1), mul_rn(DP::c3, k3));
-  s = add_rn(s, mul_rn(DP::c4, k4));
-  s = add_rn(s, mul_rn(DP::c5, k5));
-  s = add_rn(s, mul_rn(DP::c6, k6));
+  double s = add_rn(mul_rn(kRef.c[0], k1), mul_rn(kRef.c[2], k3));
+  s = add_rn(s, mul_rn(kRef.c[3], k4));
+  s = add_rn(s, mul_rn(kRef.c[4], k5));
+  s = add_rn(s, mul_rn(kRef.c[5], k6));
   return add_rn(v, mul_rn(h, s));
 }
 
 // v + h (d1 k1 + d3 k3 + d4 k4 + d5 k5 + d6 k6 + d7 k7), likewise (:299-305).
 GG_DEV double combine4(double v, double h, double k1, double k3, double k4, double k5,
                        double k6, double k7) {
-  double s = add_rn(mul_rn(DP::d1, k1), mul_rn(DP::d3, k3));
-  s = add_rn(s, mul_rn(DP::d4, k4));
-  s = add_rn(s, mul_rn(DP::d5, k5));
-  s = add_rn(s, mul_rn(DP::d6, k6));
-  s = add_rn(s, mul_rn(DP::d7, k7));
+  double s = add_rn(mul_rn(kRef.d[0], k1), mul_rn(kRef.d[2], k3));
+  s = add_rn(s, mul_rn(kRef.d[3], k4));
+  s = add_rn(s, mul_rn(kRef.d[4], k5));
+  s = add_rn(s, mul_rn(kRef.d[5], k6));
+  s = add_rn(s, mul_rn(kRef.d[6], k7));
   return add_rn(v, mul_rn(h, s));
+}
+
+// Stage S's velocity v + h sum_l b_l k_l (geodesic.rs:248-284), left to right with the
+// fused multiply-adds written out.
+template <int S, class KS>
+GG_DEV void stage_velocity(const double v[4], double h, const KS& K, double w[4]) {
+  double k[4], sum[4];
+  K.get(0, k);
+  if constexpr (S == 1) {
+    const double hb = h * kRef.b[1][0];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = fma(hb, k[i], v[i]);
+  } else {
+    double k1[4];
+    K.get(1, k1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      sum[i] = fma(kRef.b[S][0], k[i], mul_rn(kRef.b[S][1], k1[i]));
+#pragma unroll
+    for (int l = 2; l < S; ++l) {
+      K.get(l, k);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sum[i] = fma(kRef.b[S][l], k[i], sum[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = fma(h, sum[i], v[i]);
+  }
 }
 
 // One call of RK45Integrator::step (geodesic.rs:185-328) in FP64.
@@ -490,99 +528,67 @@ GG_DEV int attempt_fp64(const DevParams& P, Ray& R, const KStore& K, bool& k1_va
   if (P.has_horizon && (R.x[1] < P.rh_plus_buffer || R.x[1] < P.rh)) return kHorizon;
 
   const double h = R.h;
-  double k7[4], nv[4];
-  double r = R.x[1], th = R.x[2];
+  // The stage positions pos + (h a_s) vel lie along the step's initial
+  // velocity (geodesic.rs:248-284), uncontracted like the reference's, so the last
+  // stage's (a = 1) equals the accepted position bit for bit, which is what
+  // lets k7 serve as the next step's k1.  Rounding is monotonic, so every
+  // stage is finite with r > 0 (is_valid_position) exactly when the last one is:
+  // one test, and the stages form r and theta alone.
+  {
+    double xn[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) xn[i] = add_rn(R.x[i], mul_rn(h, R.v[i]));
+    if (!(finite4(xn[0], xn[1], xn[2], xn[3]) && xn[1] > 0.0)) {
+      R.h = h * 0.5;
+      return kContinue;
+    }
+  }
+  double k6[4], k7[4], nv[4];
   // The right-hand-side evaluations run as one loop so the RHS code (sincos,
-  // reciprocal, ~150 FP64 ops) is emitted once: unrolled, seven copies
+  // reciprocal, ~120 FP64 ops) is emitted once: unrolled, seven copies
   // overflow the instruction cache and warps stall on fetch.  The stage
-  // inputs and the k registers are selected per stage by switch arms
-  // (warp-uniform branches; all lanes of a warp run the same stage).  The
-  // last pass evaluates k6 and k7, which share the position pos6.
+  // velocities are selected per stage by switch arms (warp-uniform
+  // branches; all lanes of a warp run the same stage).  The last pass
+  // evaluates k6 and k7, which share the position pos6.
   // Warp-uniform first stage: when a refilled lane in the warp needs k1, the
   // whole warp runs stage 0 instead of the attempt diverged, but a lane whose
-  // k1 is valid keeps its own (the previous step's k7).  k7 is evaluated at
-  // another call site of the contraction, which the compiler may fuse into
-  // multiply-adds differently, so a recomputed k1 can differ from it in the
-  // last bit; overwriting it would make a ray's result depend on which rays
-  // share its warp.
+  // k1 is valid keeps its own (the previous step's k7), so that a ray's
+  // result does not depend on which rays share its warp.
   const int s_first = __any_sync(__activemask(), !k1_valid) ? 0 : 1;
 #pragma unroll 1
   for (int s = s_first; s < 6; ++s) {
-    double w[4];
+    double w[4], a[4];
     switch (s) {
       case 0:
 #pragma unroll
         for (int i = 0; i < 4; ++i) w[i] = R.v[i];
         break;
-      case 1:
-        if (!stage_pos(R, h * DP::a2, r, th)) { R.h = h * 0.5; return kContinue; }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) w[i] = R.v[i] + (h * DP::b21) * K(0, i);
-        break;
-      case 2:
-        if (!stage_pos(R, h * DP::a3, r, th)) { R.h = h * 0.5; return kContinue; }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) w[i] = R.v[i] + h * (DP::b31 * K(0, i) + DP::b32 * K(1, i));
-        break;
-      case 3:
-        if (!stage_pos(R, h * DP::a4, r, th)) { R.h = h * 0.5; return kContinue; }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          w[i] = R.v[i] + h * (DP::b41 * K(0, i) + DP::b42 * K(1, i) + DP::b43 * K(2, i));
-        break;
-      case 4:
-        if (!stage_pos(R, h * DP::a5, r, th)) { R.h = h * 0.5; return kContinue; }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          w[i] = R.v[i] +
-                 h * (DP::b51 * K(0, i) + DP::b52 * K(1, i) + DP::b53 * K(2, i) + DP::b54 * K(3, i));
-        break;
-      default:
-        if (!stage_pos(R, h, r, th)) { R.h = h * 0.5; return kContinue; }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          w[i] = R.v[i] + h * (DP::b61 * K(0, i) + DP::b62 * K(1, i) + DP::b63 * K(2, i) +
-                               DP::b64 * K(3, i) + DP::b65 * K(4, i));
-        break;
+      case 1: stage_velocity<1>(R.v, h, K, w); break;
+      case 2: stage_velocity<2>(R.v, h, K, w); break;
+      case 3: stage_velocity<3>(R.v, h, K, w); break;
+      case 4: stage_velocity<4>(R.v, h, K, w); break;
+      default: stage_velocity<5>(R.v, h, K, w); break;
     }
+    const double ha = h * kRef.a[s];  // a[0] = 0, a[5] = 1
     Geometry<METRIC, kStepperReference> G;
-    G.at(P, r, th);
-    double a[4];
+    G.at(P, add_rn(R.x[1], mul_rn(ha, R.v[1])), add_rn(R.x[2], mul_rn(ha, R.v[2])));
     G.accel(w, a);
-    switch (s) {
-      case 0:
-        if (!k1_valid) {
+    if (s == 5) {
+      double k[5][4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) K(0, i) = a[i];
-          k1_valid = true;  // a rejected attempt leaves the state, so k1 stays
-        }
-        break;
-      case 1:
+      for (int l = 0; l < 5; ++l)
+        if (l != 1) K.get(l, k[l]);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) K(1, i) = a[i];
-        break;
-      case 2:
-#pragma unroll
-        for (int i = 0; i < 4; ++i) K(2, i) = a[i];
-        break;
-      case 3:
-#pragma unroll
-        for (int i = 0; i < 4; ++i) K(3, i) = a[i];
-        break;
-      case 4:
-#pragma unroll
-        for (int i = 0; i < 4; ++i) K(4, i) = a[i];
-        break;
-      default:
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          K(5, i) = a[i];
-          nv[i] = combine5(R.v[i], h, K(0, i), K(2, i), K(3, i), K(4, i), K(5, i));
-        }
-        G.accel(nv, k7);  // k7 at (pos6, new_vel), geodesic.rs:298
-        break;
+      for (int i = 0; i < 4; ++i) {
+        k6[i] = a[i];
+        nv[i] = combine5(R.v[i], h, k[0][i], k[2][i], k[3][i], k[4][i], k6[i]);
+      }
+      G.accel(nv, k7);  // k7 at (pos6, new_vel), geodesic.rs:298
+    } else if (s > 0 || !k1_valid) {
+      K.set(s, a);
     }
   }
+  k1_valid = true;  // a rejected attempt leaves the state, so k1 stays
 
   // err = |new_vel - vel_err| (geodesic.rs:299-308).  The two vectors agree
   // to ~tol, so err is their last few bits: both are formed exactly as the
@@ -595,7 +601,7 @@ GG_DEV int attempt_fp64(const DevParams& P, Ray& R, const KStore& K, bool& k1_va
   double d[4], sc[4], ssum = 0.0;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const double ve = combine4(R.v[i], h, K(0, i), K(2, i), K(3, i), K(4, i), K(5, i), k7[i]);
+    const double ve = combine4(R.v[i], h, K(0, i), K(2, i), K(3, i), K(4, i), k6[i], k7[i]);
     d[i] = sub_rn(nv[i], ve);
   }
   if (P.rtol > 0.0) {
@@ -641,10 +647,7 @@ GG_DEV int attempt_fp64(const DevParams& P, Ray& R, const KStore& K, bool& k1_va
   R.lam = add_rn(R.lam, h);
   const bool reflected = R.x[2] < 0.0 || R.x[2] > kPi;
   normalize_coords(R.x);
-  if (!reflected) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) K(0, i) = k7[i];
-  }
+  if (!reflected) K.set(0, k7);
   k1_valid = !reflected;
   accepted = true;
   h_used = h;
@@ -726,6 +729,53 @@ struct StepEnd {
   double xraw[4];  // new position before angle normalisation
 };
 
+// Stage S's inputs x + h a_S v + h^2 sum_l Abar k_l and v + h sum_l B k_l, the sums in
+// the order of l.  Stages 1-5 form r and theta alone of the position (the
+// metric does not depend on t and phi), and leave out its zero
+// coefficient Abar[S][S-1].
+template <int S, class KS>
+GG_DEV void stage_state(const Ray& R, double h, double hh, const KS& K, double px[4],
+                        double pw[4]) {
+  const double ha = h * kDP.A[S];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (S == 6 || i == 1 || i == 2) px[i] = fma(ha, R.v[i], R.x[i]);
+    pw[i] = R.v[i];
+  }
+#pragma unroll
+  for (int l = 0; l < S; ++l) {
+    double k[4];
+    K.get(l, k);
+    const double cv = h * kDP.B[S][l];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) pw[i] = fma(cv, k[i], pw[i]);
+    if (S == 6 || l < S - 1) {
+      const double cb = hh * kDP.Abar[S][l];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (S == 6 || i == 1 || i == 2) px[i] = fma(cb, k[i], px[i]);
+    }
+  }
+}
+
+// ex += sum_l Ebar_l k_l, ev += sum_l E_l k_l over the seven stages, in order.
+template <int L, class KS>
+GG_DEV void error_sums_fp64(const KS& K, double ex[4], double ev[4]) {
+  if constexpr (L < 7) {
+    constexpr bool has_x = make_dp_table().Ebar[L] != 0.0, has_v = make_dp_table().E[L] != 0.0;
+    if constexpr (has_x || has_v) {
+      double k[4];
+      K.get(L, k);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if constexpr (has_x) ex[i] = fma(kDP.Ebar[L], k[i], ex[i]);
+        if constexpr (has_v) ev[i] = fma(kDP.E[L], k[i], ev[i]);
+      }
+    }
+    error_sums_fp64<L + 1>(K, ex, ev);
+  }
+}
+
 // One full Dormand-Prince attempt in FP64.  Same contract as attempt_fp64;
 // with k1_valid the previous step's last stage (K(6, .), evaluated at the
 // accepted state) is copied to K(0, .) first.  KS is where the stage
@@ -738,8 +788,9 @@ GG_DEV int attempt_dp45_fp64(const DevParams& P, Ray& R, const KS& K, bool& k1_v
   if (R.x[1] > P.max_radius) return kEscaped;
   if (P.has_horizon && (R.x[1] < P.rh_plus_buffer || R.x[1] < P.rh)) return kHorizon;
   if (k7_pending) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) K(0, i) = K(6, i);
+    double k[4];
+    K.get(6, k);
+    K.set(0, k);
     k7_pending = false;
   }
   const double h = R.h, hh = h * h;
@@ -747,57 +798,44 @@ GG_DEV int attempt_dp45_fp64(const DevParams& P, Ray& R, const KS& K, bool& k1_v
   const int s_first = __any_sync(__activemask(), !k1_valid) ? 0 : 1;
 #pragma unroll 1
   for (int s = s_first; s < 7; ++s) {
-    double px[4], pw[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      px[i] = R.x[i];
-      pw[i] = R.v[i];
-    }
-    if (s > 0) {
-      const double ha = h * kDP.A[s];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) px[i] = fma(ha, R.v[i], px[i]);
-#pragma unroll 1
-      for (int l = 0; l < s; ++l) {
-        const double cb = hh * kDP.Abar[s][l], cv = h * kDP.B[s][l];
+    double px[4], pw[4], a[4];
+    switch (s) {  // the last pass leaves the step's end in (px, pw)
+      case 0:
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const double kl = K(l, i);
-          px[i] = fma(cb, kl, px[i]);
-          pw[i] = fma(cv, kl, pw[i]);
+          px[i] = R.x[i];
+          pw[i] = R.v[i];
         }
-      }
-      if (!(finite4(px[0], px[1], px[2], px[3]) && px[1] > 0.0)) {
-        R.h = h * 0.5;
-        return kContinue;
-      }
+        break;
+      case 1: stage_state<1>(R, h, hh, K, px, pw); break;
+      case 2: stage_state<2>(R, h, hh, K, px, pw); break;
+      case 3: stage_state<3>(R, h, hh, K, px, pw); break;
+      case 4: stage_state<4>(R, h, hh, K, px, pw); break;
+      case 5: stage_state<5>(R, h, hh, K, px, pw); break;
+      default:
+        stage_state<6>(R, h, hh, K, px, pw);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          xn[i] = px[i];
+          vn[i] = pw[i];
+        }
+        if (!(isfinite(px[0]) && isfinite(px[3]))) px[1] = -1.0;
+        break;
+    }
+    // is_valid_position; t and phi overflow only with a stage derivative that is not
+    // finite, which reaches r by the next stage, so they are tested at the last
+    if (s > 0 && !(isfinite(px[1]) && isfinite(px[2]) && px[1] > 0.0)) {
+      R.h = h * 0.5;
+      return kContinue;
     }
     Geometry<METRIC, kStepperDP45> G;
     G.at(P, px[1], px[2]);
-    double a[4];
     G.accel(pw, a);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) K(s, i) = a[i];
-    if (s == 6) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        xn[i] = px[i];
-        vn[i] = pw[i];
-      }
-    }
+    K.set(s, a);
   }
   // embedded error of positions (h^2 sum Ebar k) and velocities (h sum E k)
   double ex[4] = {0.0, 0.0, 0.0, 0.0}, ev[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 1
-  for (int l = 0; l < 7; ++l) {
-    const double eb = kDP.Ebar[l], e = kDP.E[l];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const double kl = K(l, i);
-      ex[i] = fma(eb, kl, ex[i]);
-      ev[i] = fma(e, kl, ev[i]);
-    }
-  }
+  error_sums_fp64<0>(K, ex, ev);
   // as in attempt_fp64: an attempt at max_step whose errors are all well
   // inside their scales is accepted and keeps max_step
   bool steady = h == P.max_step;

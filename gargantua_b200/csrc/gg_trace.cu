@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kTraceBlock,
       SRC == kSrcQueue ? (ctl->queued < O.queue_cap ? ctl->queued : O.queue_cap) : P.n_rays;
   unsigned long long* const head = SRC == kSrcQueue ? &ctl->next_queued : &ctl->next_ray;
   __shared__ BlockStats bs;
-  __shared__ double k_smem[7][4][kTraceBlock];  // stage derivatives, see KStore
+  __shared__ double2 k_smem[7][2][kTraceBlock];  // stage derivatives, see KStore
   const KStore K{k_smem};
   if (threadIdx.x < sizeof(BlockStats) / 8)
     reinterpret_cast<unsigned long long*>(&bs)[threadIdx.x] = 0ull;
