@@ -39,6 +39,8 @@ struct gg_ctx {
   size_t queue_cap = 0;
   void* ret = nullptr;             // mixed form: rays the FP64 pass hands back
   size_t ret_cap = 0;
+  void* chain = nullptr;           // FP64 renders: rays handed to the group pass
+  size_t chain_cap = 0;
   // batched renders: scene table (device and pinned host mirror), kernel
   // variant, and the cached graph of the last batch shape
   void* batch_dev = nullptr;
@@ -486,9 +488,17 @@ int enqueue(gg_ctx* ctx, const DevParams& P, DevOutputs O, bool want_image,
   const cudaError_t oe = mixed ? gg::mixed_occupancy(P, &bps) : gg::trace_occupancy(P, &bps);
   if (oe != cudaSuccess || bps < 1) return GG_ERR_CUDA;
   uint64_t grid = (uint64_t)ctx->sms * (uint64_t)bps;
-  const uint64_t need_blocks = (P.n_rays + gg::kTraceBlock - 1) / gg::kTraceBlock;
+  const uint64_t need_blocks =
+      mixed ? (P.n_rays + gg::kTraceBlock - 1) / gg::kTraceBlock : gg::trace_blocks(P);
   if (grid > need_blocks) grid = need_blocks;
   if (grid < 1) grid = 1;
+  O.chain = nullptr;
+  O.chain_cap = mixed ? 0u : (uint32_t)gg::chain_capacity(P, (int)grid);
+  if (O.chain_cap) {
+    const int st = grow(&ctx->chain, &ctx->chain_cap, sizeof(gg::ChainRay) * O.chain_cap);
+    if (st != GG_OK) return st;
+    O.chain = static_cast<gg::ChainRay*>(ctx->chain);
+  }
   int qbps = 0, rbps = 0;
   if (mixed && (gg::queue_trace_occupancy(P, &qbps) != cudaSuccess || qbps < 1))
     return GG_ERR_CUDA;
@@ -510,7 +520,8 @@ int enqueue(gg_ctx* ctx, const DevParams& P, DevOutputs O, bool want_image,
           gg::launch_queue_trace(P, O, ctx->ctl, ctx->sms * qbps, stream) != cudaSuccess)
         return GG_ERR_CUDA;
     }
-  } else if (gg::launch_trace(P, O, ctx->ctl, (int)grid, stream) != cudaSuccess) {
+  } else if (gg::launch_trace(P, O, ctx->ctl, (int)grid, stream) != cudaSuccess ||
+             (O.chain && gg::launch_group(P, O, ctx->ctl, ctx->sms, stream) != cudaSuccess)) {
     return GG_ERR_CUDA;
   }
   if (cudaEventRecord(ctx->ev_stop, stream) != cudaSuccess) return GG_ERR_CUDA;
@@ -923,6 +934,7 @@ GG_API int gg_destroy(gg_ctx* c) {
   if (c->staging) cudaFree(c->staging);
   if (c->queue) cudaFree(c->queue);
   if (c->ret) cudaFree(c->ret);
+  if (c->chain) cudaFree(c->chain);
   if (c->batch_exec) cudaGraphExecDestroy(c->batch_exec);
   if (c->batch_dev) cudaFree(c->batch_dev);
   if (c->batch_host) cudaFreeHost(c->batch_host);

@@ -117,7 +117,6 @@ template <class T>
 struct SchwGeoT {
   T g_t_tr, g_r_tt, g_r_thth, g_r_phph, ir, g_th_phph, g_ph_thph;
 };
-using SchwGeo = SchwGeoT<double>;
 
 template <class T>
 GG_DEV SchwGeoT<T> schw_geometry(T rs, T r, T s, T c) {
@@ -232,6 +231,44 @@ GG_DEV void kerr_contract64(const KerrGeo64& G, const double v[4], double acc[4]
   acc[2] = -G.n_thth * y;
 }
 
+// Schwarzschild likewise: the pair above with its halves and doubles taken out
+// and nvcc's fused multiply-adds written out, the same to the last bit.
+struct SchwGeo64 {
+  double q, g_r_tt, rmrs, g_r_phph, two_ir, g_th_phph, two_ph_thph;  // q = 2 g_t_tr
+};
+
+GG_DEV SchwGeo64 schw_geometry64(const DevParams& P, double r, double s, double c) {
+  SchwGeo64 G;
+  G.rmrs = r - P.rs;
+  const double rr = r * G.rmrs;
+  const double R = 1.0 / (rr * s);  // 1 / (r (r - rs) sin)
+  const double ifd = s * R;         // 1 / (r (r - rs))
+  const double ir = G.rmrs * ifd;   // 1 / r
+  const double is = rr * R;         // 1 / sin
+  G.q = P.rs * ifd;
+  G.g_r_tt = P.mass * G.rmrs * (ir * ir * ir);
+  G.g_r_phph = G.rmrs * s * s;  // negated, like rmrs = -g_r_thth and g_th_phph
+  G.two_ir = ir + ir;
+  G.g_th_phph = s * c;
+  const double cis = c * is;
+  G.two_ph_thph = cis + cis;
+  return G;
+}
+
+// K7: the reference step's k7, whose r row nvcc fused the other way round.
+template <bool K7>
+GG_DEV void schw_contract64(const SchwGeo64& G, const double v[4], double a[4]) {
+  const double vt = v[0], vr = v[1], vth = v[2], vph = v[3];
+  a[0] = -(G.q * vt * vr);
+  const double tr = mul_rn(0.5 * G.q, vr), tt = mul_rn(G.g_r_tt, vt);
+  double x = K7 ? fma(-tt, vt, mul_rn(tr, vr)) : fma(tr, vr, -mul_rn(tt, vt));
+  x = fma(mul_rn(G.rmrs, vth), vth, x);
+  a[1] = fma(mul_rn(G.g_r_phph, vph), vph, x);
+  const double b = mul_rn(-G.two_ir, vr);
+  a[2] = fma(b, vth, mul_rn(mul_rn(G.g_th_phph, vph), vph));
+  a[3] = fma(b, vph, -mul_rn(mul_rn(G.two_ph_thph, vth), vph));
+}
+
 template <int METRIC, int STEPPER>
 struct Geometry;
 
@@ -243,18 +280,24 @@ struct Geometry<kMetricKerr, STEPPER> {
     sincos(th, &s, &c);
     g = kerr_geometry64(P, fmax(r, 1e-10), s, c);
   }
-  GG_DEV void accel(const double v[4], double a[4]) const { kerr_contract64<STEPPER>(g, v, a); }
+  template <bool K7 = false>
+  GG_DEV void accel(const double v[4], double a[4]) const {
+    kerr_contract64<STEPPER>(g, v, a);
+  }
 };
 
 template <int STEPPER>
 struct Geometry<kMetricSchwarzschild, STEPPER> {
-  SchwGeo g;
+  SchwGeo64 g;
   GG_DEV void at(const DevParams& P, double r, double th) {
     double s, c;
     sincos(th, &s, &c);
-    g = schw_geometry<double>(P.rs, fmax(r, 1e-10), s, c);
+    g = schw_geometry64(P, fmax(r, 1e-10), s, c);
   }
-  GG_DEV void accel(const double v[4], double a[4]) const { schw_contract<double>(g, v, a); }
+  template <bool K7 = false>
+  GG_DEV void accel(const double v[4], double a[4]) const {
+    schw_contract64<K7>(g, v, a);
+  }
 };
 
 // ---------------------------------------------------------------------------
@@ -262,7 +305,7 @@ struct Geometry<kMetricSchwarzschild, STEPPER> {
 // accepted step by the disks, not per stage).
 // ---------------------------------------------------------------------------
 struct Gmet {
-  double tt, rr, thth, phph, tph;
+  double tt, phph, tph;
 };
 
 template <int METRIC>
@@ -273,19 +316,13 @@ GG_DEV Gmet metric_tensor(const DevParams& P, double r_in, double th) {
   if (METRIC == kMetricKerr) {  // kerr.rs:61-94
     const double m = P.mass, a = P.spin, a2 = a * a;
     const double c = cos(th);
-    const double sig = r * r + a * a * c * c;
-    const double del = r * r - 2.0 * m * r + a * a;
+    const double sig = fma(r, r, mul_rn(a2 * c, c));
     const double sin2 = s * s;
-    g.tt = -(1.0 - 2.0 * m * r / sig);
-    g.rr = sig / del;
-    g.thth = sig;
-    g.phph = (r * r + a2 + 2.0 * m * a2 * r * sin2 / sig) * sin2;
+    g.tt = -sub_rn(1.0, 2.0 * m * r / sig);
+    g.phph = add_rn(fma(r, r, a2), 2.0 * m * a2 * r * sin2 / sig) * sin2;
     g.tph = -2.0 * m * a * r * sin2 / sig;
   } else {  // schwarzschild.rs:26-43
-    const double f = 1.0 - P.rs / r;
-    g.tt = -f;
-    g.rr = 1.0 / f;
-    g.thth = r * r;
+    g.tt = -sub_rn(1.0, P.rs / r);
     g.phph = r * r * s * s;
     g.tph = 0.0;
   }
@@ -298,7 +335,7 @@ GG_DEV Gmet metric_tensor(const DevParams& P, double r_in, double th) {
 template <int METRIC>
 GG_DEV double redshift_factor(const DevParams& P, double r, double th, const double p[4]) {
   const Gmet g = metric_tensor<METRIC>(P, r, th);
-  const double p_t = g.tt * p[0] + g.tph * p[3];
+  const double p_t = fma(g.tph, p[3], mul_rn(g.tt, p[0]));
   const double e_obs = fmax(-p_t / P.sqrt_neg_gtt_obs, 0.0);
   bool has_orbit;
   double omega = 0.0;
@@ -306,7 +343,7 @@ GG_DEV double redshift_factor(const DevParams& P, double r, double th, const dou
     has_orbit = r > 0.0;
     if (has_orbit) {
       const double sqrt_m = sqrt(P.mass);
-      omega = sqrt_m / (pow(r, 1.5) + P.spin * sqrt_m);
+      omega = sqrt_m / fma(P.spin, sqrt_m, pow(r, 1.5));
     }
   } else {
     has_orbit = !(r <= 3.0 * P.mass);
@@ -315,13 +352,13 @@ GG_DEV double redshift_factor(const DevParams& P, double r, double th, const dou
   double e_emit = 0.0;
   bool used_orbit = false;
   if (has_orbit) {
-    const Gmet go = metric_tensor<METRIC>(P, r, th);
-    const double denom = -(go.tt + 2.0 * go.tph * omega + go.phph * omega * omega);
+    const double denom =
+        -fma(mul_rn(g.phph, omega), omega, fma(2.0 * g.tph, omega, g.tt));
     if (denom > 0.0 && isfinite(denom)) {
       const double u_t = 1.0 / sqrt(denom);
       const double u_p = omega * u_t;
-      const double p_phi = g.tph * p[0] + g.phph * p[3];
-      e_emit = fmax(-(p_t * u_t + p_phi * u_p), 0.0);
+      const double p_phi = fma(g.tph, p[0], mul_rn(g.phph, p[3]));
+      e_emit = fmax(-fma(p_t, u_t, mul_rn(p_phi, u_p)), 0.0);
       used_orbit = true;
     }
   }
@@ -511,6 +548,60 @@ GG_DEV void stage_velocity(const double v[4], double h, const KS& K, double w[4]
   }
 }
 
+// The end of a reference attempt: new velocity nv, its embedded error d
+// (geodesic.rs:306-327).  The acceptance test and the step-size law; advances
+// the ray (position not yet normalised) and returns true if the step stands.
+GG_DEV bool end_attempt_fp64(const DevParams& P, Ray& R, const double nv[4], const double d[4]) {
+  const double h = R.h;
+  // `steady`: the step is max_step already and every component's error is
+  // within kSteadyErr of its scale, so the step is accepted and the law's
+  // clamp gives max_step again: the norm's divisions and root are not needed.
+  bool steady = h == P.max_step;
+  double sc[4], ssum = 0.0;
+  if (P.rtol > 0.0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      sc[i] = add_rn(P.atol, mul_rn(P.rtol, fmax(fabs(R.v[i]), fabs(nv[i]))));
+      steady = steady && fabs(d[i]) <= kSteadyErr * sc[i];
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ssum = add_rn(ssum, mul_rn(d[i], d[i]));
+    steady = steady && ssum < (kSteadyErr * kSteadyErr * 0.98) * P.tolerance * P.tolerance;
+  }
+  if (!steady) {
+    double err, tol;
+    if (P.rtol > 0.0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const double q = __ddiv_rn(d[i], sc[i]);
+        ssum = add_rn(ssum, mul_rn(q, q));
+      }
+      err = __dsqrt_rn(mul_rn(ssum, 0.25));
+      tol = 1.0;
+    } else {
+      err = __dsqrt_rn(ssum);
+      tol = P.tolerance;
+    }
+    if (!(err < tol || h <= P.min_step)) {
+      // (tol/err)^0.25 as two correctly rounded square roots
+      R.h = fmax(h * 0.9 * sqrt(sqrt(tol / err)), P.min_step);
+      return false;
+    }
+    if (err > 0.0) {
+      double hn = h * 0.9 * fifth_root(tol / err);
+      hn = hn < P.min_step ? P.min_step : (hn > P.max_step ? P.max_step : hn);
+      R.h = hn;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) R.x[i] = add_rn(R.x[i], mul_rn(h, R.v[i]));  // geodesic.rs:312
+#pragma unroll
+  for (int i = 0; i < 4; ++i) R.v[i] = nv[i];
+  R.lam = add_rn(R.lam, h);
+  return true;
+}
+
 // One call of RK45Integrator::step (geodesic.rs:185-328) in FP64.
 // Returns the StepResult; `accepted` and `h_used` describe an advance.
 template <int METRIC>
@@ -583,7 +674,7 @@ GG_DEV int attempt_fp64(const DevParams& P, Ray& R, const KStore& K, bool& k1_va
         k6[i] = a[i];
         nv[i] = combine5(R.v[i], h, k[0][i], k[2][i], k[3][i], k[4][i], k6[i]);
       }
-      G.accel(nv, k7);  // k7 at (pos6, new_vel), geodesic.rs:298
+      G.template accel<true>(nv, k7);  // k7 at (pos6, new_vel), geodesic.rs:298
     } else if (s > 0 || !k1_valid) {
       K.set(s, a);
     }
@@ -594,60 +685,127 @@ GG_DEV int attempt_fp64(const DevParams& P, Ray& R, const KStore& K, bool& k1_va
   // to ~tol, so err is their last few bits: both are formed exactly as the
   // reference groups them, without fused multiply-adds, so that only the
   // (much smaller) differences in the k's reach the step-size law.
-  // `steady`: the step is max_step already and every component's error is
-  // within kSteadyErr of its scale, so the step is accepted and the law's
-  // clamp gives max_step again: the norm's divisions and root are not needed.
-  bool steady = h == P.max_step;
-  double d[4], sc[4], ssum = 0.0;
+  double d[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const double ve = combine4(R.v[i], h, K(0, i), K(2, i), K(3, i), K(4, i), k6[i], k7[i]);
     d[i] = sub_rn(nv[i], ve);
   }
-  if (P.rtol > 0.0) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      sc[i] = add_rn(P.atol, mul_rn(P.rtol, fmax(fabs(R.v[i]), fabs(nv[i]))));
-      steady = steady && fabs(d[i]) <= kSteadyErr * sc[i];
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) ssum = add_rn(ssum, mul_rn(d[i], d[i]));
-    steady = steady && ssum < (kSteadyErr * kSteadyErr * 0.98) * P.tolerance * P.tolerance;
-  }
-  if (!steady) {
-    double err, tol;
-    if (P.rtol > 0.0) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const double q = __ddiv_rn(d[i], sc[i]);
-        ssum = add_rn(ssum, mul_rn(q, q));
-      }
-      err = __dsqrt_rn(mul_rn(ssum, 0.25));
-      tol = 1.0;
-    } else {
-      err = __dsqrt_rn(ssum);
-      tol = P.tolerance;
-    }
-    if (!(err < tol || h <= P.min_step)) {
-      // (tol/err)^0.25 as two correctly rounded square roots
-      R.h = fmax(h * 0.9 * sqrt(sqrt(tol / err)), P.min_step);
-      return kContinue;
-    }
-    if (err > 0.0) {
-      double hn = h * 0.9 * fifth_root(tol / err);
-      hn = hn < P.min_step ? P.min_step : (hn > P.max_step ? P.max_step : hn);
-      R.h = hn;
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) R.x[i] = add_rn(R.x[i], mul_rn(h, R.v[i]));  // geodesic.rs:312
-#pragma unroll
-  for (int i = 0; i < 4; ++i) R.v[i] = nv[i];
-  R.lam = add_rn(R.lam, h);
+  if (!end_attempt_fp64(P, R, nv, d)) return kContinue;
   const bool reflected = R.x[2] < 0.0 || R.x[2] > kPi;
   normalize_coords(R.x);
   if (!reflected) K.set(0, k7);
+  k1_valid = !reflected;
+  accepted = true;
+  h_used = h;
+  return kContinue;
+}
+
+// ---------------------------------------------------------------------------
+// The same attempt by a group of kGroupLanes lanes that share one ray.
+//
+// A ray alone in its warp takes an attempt in about 3 us: five geometries and
+// six contractions, one after the other, each operation waiting for the last.
+// But the reference step's stage positions do not depend on the stage derivatives
+// (they lie along the initial velocity), so the group's lanes take one stage's
+// geometry each, at the same time, and only the contractions remain in
+// sequence: lane s contracts stage s and passes k_(s+1) on by shuffles.  Every lane
+// carries the whole ray and does the rest (sums, error, step law) redundantly.
+// Operations and their order per value are attempt_fp64's, so the bits are too.
+// Fewer rays are in flight than with a lane each (about 5 G attempts/s at full
+// occupancy against 12.8 G), so this form is for few rays: small renders and
+// the last rays of large ones (gg_trace.cu).  Measured on a 32x24 picture
+// (768 rays, up to 351 attempts): 1.01 ms with a lane per ray, 0.47 ms so.
+// ---------------------------------------------------------------------------
+constexpr int kGroupLanes = 8;  // lanes 0..5 take stage 0..5, the last two copy lane 5
+
+struct GroupRole {
+  unsigned mask;   // the group's lanes of the warp
+  double a, b[5];  // this lane's stage: node and velocity weights
+  GG_DEV static GroupRole at(unsigned lane) {
+    GroupRole g;
+    const int s = (int)(lane % kGroupLanes);
+    const int st = s < 5 ? s : 5;
+    g.mask = ((1u << kGroupLanes) - 1u) << (lane & ~(unsigned)(kGroupLanes - 1));
+    g.a = kRef.a[st];
+#pragma unroll
+    for (int l = 0; l < 5; ++l) g.b[l] = kRef.b[st][l];
+    return g;
+  }
+  // lane `src` of the group's copy of k
+  GG_DEV void share(double k[4], int src) const {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) k[i] = __shfl_sync(mask, k[i], src, kGroupLanes);
+  }
+};
+
+template <int METRIC>
+GG_DEV int attempt_fp64_group(const DevParams& P, Ray& R, const GroupRole& role, double k1[4],
+                              bool& k1_valid, bool& accepted, double& h_used) {
+  accepted = false;
+  if (R.x[1] > P.max_radius) return kEscaped;
+  if (P.has_horizon && (R.x[1] < P.rh_plus_buffer || R.x[1] < P.rh)) return kHorizon;
+
+  const double h = R.h;
+  {
+    double xn[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) xn[i] = add_rn(R.x[i], mul_rn(h, R.v[i]));
+    if (!(finite4(xn[0], xn[1], xn[2], xn[3]) && xn[1] > 0.0)) {
+      R.h = h * 0.5;
+      return kContinue;
+    }
+  }
+  const double ha = h * role.a;
+  Geometry<METRIC, kStepperReference> G;
+  G.at(P, add_rn(R.x[1], mul_rn(ha, R.v[1])), add_rn(R.x[2], mul_rn(ha, R.v[2])));
+  if (!k1_valid) {
+    G.accel(R.v, k1);
+    role.share(k1, 0);
+    k1_valid = true;
+  }
+  // stage sums of this lane's stage, and both solutions' sums, as each k arrives
+  double w[4], k[4], t[4], sc[4], sd[4];
+  const double hb = h * role.b[0];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    w[i] = fma(hb, k1[i], R.v[i]);
+    sc[i] = mul_rn(kRef.c[0], k1[i]);
+    sd[i] = mul_rn(kRef.d[0], k1[i]);
+  }
+#pragma unroll
+  for (int s = 1; s < 6; ++s) {  // k_(s+1), contracted by lane s
+    G.accel(w, k);
+    role.share(k, s);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (s > 1) {
+        sc[i] = add_rn(sc[i], mul_rn(kRef.c[s], k[i]));
+        sd[i] = add_rn(sd[i], mul_rn(kRef.d[s], k[i]));
+      }
+      if (s < 5) {
+        t[i] = s == 1 ? fma(role.b[0], k1[i], mul_rn(role.b[1], k[i])) : fma(role.b[s], k[i], t[i]);
+        w[i] = fma(h, t[i], R.v[i]);
+      }
+    }
+  }
+  double nv[4], d[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) nv[i] = add_rn(R.v[i], mul_rn(h, sc[i]));
+  G.template accel<true>(nv, k);  // k7, by the lanes at pos6
+  role.share(k, 5);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double ve = add_rn(R.v[i], mul_rn(h, add_rn(sd[i], mul_rn(kRef.d[6], k[i]))));
+    d[i] = sub_rn(nv[i], ve);
+  }
+  if (!end_attempt_fp64(P, R, nv, d)) return kContinue;
+  const bool reflected = R.x[2] < 0.0 || R.x[2] > kPi;
+  normalize_coords(R.x);
+  if (!reflected) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) k1[i] = k[i];
+  }
   k1_valid = !reflected;
   accepted = true;
   h_used = h;

@@ -41,6 +41,7 @@ constexpr int kTraceMinBlocksKerrChain = 4;
 #endif
 constexpr int kTraceMinBlocksSchw = 4;
 #endif
+constexpr int kTraceMinBlocksGroup = 3;  // 168 registers: no spills, latency is all that counts
 
 // Resident CTAs per SM the mixed-precision trace kernel is budgeted for: its
 // camera pass (8, 64 registers: throughput), and its pass over the rays the
@@ -58,8 +59,17 @@ constexpr int kMixedMinBlocksReturned = GG_MIXED_RET_MIN_BLOCKS;
 constexpr int kMixedMinBlocksReturned = 4;
 #endif
 
-// Resident CTAs per SM of the trace kernel `P` selects.
+// Resident CTAs per SM of the trace kernel `P` selects, and the CTAs that
+// give each of its rays a place at once.
 cudaError_t trace_occupancy(const DevParams& P, int* blocks_per_sm);
+uint64_t trace_blocks(const DevParams& P);
+
+// The group pass over the rays that launch_trace's draining warps leave in
+// O.chain (chain_capacity entries for `grid` CTAs of that launch; 0: the
+// render has no such pass and O.chain stays null).
+int chain_capacity(const DevParams& P, int grid);
+cudaError_t launch_group(const DevParams& P, const DevOutputs& O, DevControl* ctl, int sms,
+                         cudaStream_t stream);
 
 // Persistent trace over P.n_rays samples; `grid` CTAs of kTraceBlock threads.
 cudaError_t launch_trace(const DevParams& P, const DevOutputs& O, DevControl* ctl, int grid,

@@ -119,7 +119,7 @@ extern "C" GG_API int gg_render_device_noalloc(const gg_metric_t* metric,
   int bps = 0;
   if (gg::trace_occupancy(P, &bps) != cudaSuccess || bps < 1) return cuda_failed();
   uint64_t grid = (uint64_t)sms * (uint64_t)bps;
-  const uint64_t need_blocks = (P.n_rays + gg::kTraceBlock - 1) / gg::kTraceBlock;
+  const uint64_t need_blocks = gg::trace_blocks(P);
   if (grid > need_blocks) grid = need_blocks;
   if (grid < 1) grid = 1;
   if (gg::launch_trace(P, O, ctl, (int)grid, s) != cudaSuccess) return cuda_failed();

@@ -143,7 +143,23 @@ struct DevOutputs {
   struct Ckpt* ckpt;         // differentiable render: ckpt_per_ray entries per ray
   struct DiffRay* diff_rays;
   uint32_t ckpt_per_ray;
-  uint32_t pad_ckpt;
+  // FP64 renders with the reference's step: rays a draining warp hands to the
+  // group pass (gg_trace.cu)
+  uint32_t chain_cap;
+  struct ChainRay* chain;
+};
+
+// A ray of an FP64 render on its way to the group pass: its state between two
+// attempts, with k1 = a(x, v) if it is known and the disk's accumulators.
+struct ChainRay {
+  double x[4];
+  double v[4];
+  double k1[4];
+  double h, lam;
+  double inten, trans;
+  uint64_t idx;
+  uint32_t n_att, n_acc;
+  uint32_t k1_valid, crossed;
 };
 
 // A ray the mixed-precision pass hands to the FP64 pass (its state at the
@@ -213,6 +229,8 @@ struct DevControl {
   unsigned long long returned;       // rays the FP64 pass handed back to the mixed form
   unsigned long long next_returned;  // the mixed form's head on that queue
   unsigned long long band_total;     // hand-offs to the FP64 pass of earlier rounds
+  unsigned long long chained;        // rays handed to the group pass
+  unsigned long long next_chained;   // the group pass's queue head
 };
 
 }  // namespace gg

@@ -63,6 +63,16 @@ __device__ __noinline__ void hand_back(const DevOutputs& O, DevControl* ctl, Ray
   q.scene = scene;
 }
 
+// Writes a ray to the group pass's queue; false (the ray stays) if it is full.
+// Out of line: at most kHandLanes times per warp.
+__device__ __noinline__ bool hand_to_group(const DevOutputs& O, DevControl* ctl,
+                                           const ChainRay& q) {
+  const unsigned long long slot = atomicAdd(&ctl->chained, 1ull);
+  if (slot >= O.chain_cap) return false;
+  O.chain[slot] = q;
+  return true;
+}
+
 // SRC: kSrcCamera traces the render's samples from the camera; kSrcQueue
 // finishes, in FP64, the rays the mixed-precision pass handed over (their
 // count is read from ctl->queued, which that pass wrote before this launch);
@@ -73,22 +83,40 @@ __device__ __noinline__ void hand_back(const DevOutputs& O, DevControl* ctl, Ray
 // objects first.  CKPT (kSrcCamera, Kerr, thin disk, full Dormand-Prince):
 // the differentiable render's forward, which also stores each ray's state
 // (x, v, next h) at its start and after every kCkptEvery-th accepted step it
-// survives (O.ckpt) and, when it ends, its DiffRay (O.diff_rays).
+// survives (O.ckpt) and, when it ends, its DiffRay (O.diff_rays).  GROUP
+// (kSrcCamera, the reference's step): kGroupLanes lanes share a ray
+// (attempt_fp64_group); the rays come from the group queue if there is one
+// (O.chain), else from the camera.  Without GROUP, a warp that finds no more
+// samples and has at most kHandLanes rays left hands those to that queue.
 template <int METRIC, int DISK, int STEPPER, int SRC, bool BATCH, bool SCENE, bool CKPT,
-          bool SMALL>
+          bool SMALL, bool GROUP>
 __global__ void __launch_bounds__(kTraceBlock,
-                                  METRIC != kMetricKerr                 ? kTraceMinBlocksSchw
+                                  GROUP                                 ? kTraceMinBlocksGroup
+                                  : METRIC != kMetricKerr               ? kTraceMinBlocksSchw
                                   : (SRC == kSrcQueue || CKPT || SMALL) ? kTraceMinBlocksKerrChain
                                                                         : kTraceMinBlocksKerr)
     trace_fp64_kernel(const __grid_constant__ DevParams P, const __grid_constant__ DevOutputs O,
                       DevControl* ctl, const __grid_constant__ BatchTable B) {
   const unsigned lane = threadIdx.x & 31u;
+  const bool from_chain = GROUP && O.chain != nullptr;
   const uint64_t n_src =
-      SRC == kSrcQueue ? (ctl->queued < O.queue_cap ? ctl->queued : O.queue_cap) : P.n_rays;
-  unsigned long long* const head = SRC == kSrcQueue ? &ctl->next_queued : &ctl->next_ray;
+      SRC == kSrcQueue ? (ctl->queued < O.queue_cap ? ctl->queued : O.queue_cap)
+      : from_chain     ? (ctl->chained < O.chain_cap ? ctl->chained : O.chain_cap)
+                       : P.n_rays;
+  unsigned long long* const head = SRC == kSrcQueue ? &ctl->next_queued
+                                   : from_chain     ? &ctl->next_chained
+                                                    : &ctl->next_ray;
+  // lanes that stand for a ray in the votes (one per group), and whether this
+  // one writes its ray's results
+  const unsigned ray_lanes = GROUP ? kGroupLeaders : kFull;
+  const bool writer = !GROUP || lane % kGroupLanes == 0;
+  constexpr uint32_t chunk = GROUP ? 32 / kGroupLanes : kChunk;
   __shared__ BlockStats bs;
-  __shared__ double2 k_smem[7][2][kTraceBlock];  // stage derivatives, see KStore
+  __shared__ double2 k_smem[GROUP ? 1 : 7][2][kTraceBlock];  // stage derivatives, see KStore
   const KStore K{k_smem};
+  GroupRole role;
+  double k1[4];  // GROUP: a(x, v) of the current state if k1_valid
+  if (GROUP) role = GroupRole::at(lane);
   if (threadIdx.x < sizeof(BlockStats) / 8)
     reinterpret_cast<unsigned long long*>(&bs)[threadIdx.x] = 0ull;
   __syncthreads();
@@ -129,6 +157,8 @@ __global__ void __launch_bounds__(kTraceBlock,
   uint32_t wcount = 0;
   bool wdone = false;
   unsigned budget_pending = 0;
+  constexpr bool kHandsOver =
+      STEPPER == kStepperReference && SRC == kSrcCamera && !GROUP && !CKPT && !BATCH;
 
   for (;;) {
     // ---- refill lanes whose ray finished ----------------------------------
@@ -142,7 +172,7 @@ __global__ void __launch_bounds__(kTraceBlock,
       if (wcount == 0) {
         unsigned long long b = 0;
         if (lane == 0) {
-          b = atomicAdd(head, (unsigned long long)kChunk);
+          b = atomicAdd(head, (unsigned long long)chunk);
           if (P.attempt_budget) {
             const unsigned long long used = atomicAdd(&ctl->budget_used, 0ull);
             if (used > P.attempt_budget) {
@@ -158,13 +188,37 @@ __global__ void __launch_bounds__(kTraceBlock,
         }
         wbase = b;
         const uint64_t left = n_src - b;
-        wcount = left < kChunk ? (uint32_t)left : kChunk;
+        wcount = left < chunk ? (uint32_t)left : chunk;
       }
-      const unsigned nn = (unsigned)__popc(need);
+      const unsigned nn = (unsigned)__popc(need & ray_lanes);
       const unsigned take = nn < wcount ? nn : wcount;
-      const unsigned rank = (unsigned)__popc(need & lanemask_lt());
+      const unsigned below =
+          GROUP ? (1u << (lane & ~(unsigned)(kGroupLanes - 1))) - 1u : lanemask_lt();
+      const unsigned rank = (unsigned)__popc(need & ray_lanes & below);
       if (!live && rank < take) {
-        if (SRC == kSrcQueue) {
+        inten = 0.0;
+        trans = 1.0;
+        crossed = false;
+        k1_valid = false;
+        k7_pending = false;
+        if (from_chain) {
+          const ChainRay& q = O.chain[wbase + rank];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            R.x[i] = q.x[i];
+            R.v[i] = q.v[i];
+            k1[i] = q.k1[i];
+          }
+          R.h = q.h;
+          R.lam = q.lam;
+          inten = q.inten;
+          trans = q.trans;
+          idx = q.idx;
+          n_att = q.n_att;
+          n_acc = q.n_acc;
+          k1_valid = q.k1_valid != 0u;
+          crossed = q.crossed != 0u;
+        } else if (SRC == kSrcQueue) {
           const QueuedRay& q = O.queue[wbase + rank];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -188,21 +242,39 @@ __global__ void __launch_bounds__(kTraceBlock,
           }
         }
         live = true;
-        inten = 0.0;
-        trans = 1.0;
-        crossed = false;
-        k1_valid = false;
-        k7_pending = false;
       }
       wbase += take;
       wcount -= take;
       need = __ballot_sync(kFull, !live);
     }
+    if (kHandsOver && wdone && O.chain) {
+      const unsigned left = 32u - (unsigned)__popc(need);
+      if (live && left <= kHandLanes) {
+        ChainRay q;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          q.x[i] = R.x[i];
+          q.v[i] = R.v[i];
+          q.k1[i] = K(0, i);
+        }
+        q.h = R.h;
+        q.lam = R.lam;
+        q.inten = inten;
+        q.trans = trans;
+        q.idx = idx;
+        q.n_att = n_att;
+        q.n_acc = n_acc;
+        q.k1_valid = k1_valid ? 1u : 0u;
+        q.crossed = crossed ? 1u : 0u;
+        if (hand_to_group(O, ctl, q)) live = false;
+      }
+    }
     if (!__any_sync(kFull, live)) break;
 
     // ---- advance every live ray by up to kPeriod attempts -----------------
 #pragma unroll 1
-    for (int it = 0; it < (SRC == kSrcQueue ? kQueuePeriod : kPeriod); ++it) {
+    for (int it = 0; it < (SRC == kSrcQueue ? kQueuePeriod : GROUP ? kGroupPeriod : kPeriod);
+         ++it) {
       if (!live) continue;
       // this lane's scene: the batch's entry, or the render's own parameters
       const DevParams& PL = BATCH ? B.scenes[scene].P : P;
@@ -220,6 +292,8 @@ __global__ void __launch_bounds__(kTraceBlock,
       int res;
       if (STEPPER == kStepperDP45)
         res = attempt_dp45_fp64<METRIC>(PL, R, K, k1_valid, k7_pending, acc, h_used, end);
+      else if (GROUP)
+        res = attempt_fp64_group<METRIC>(PL, R, role, k1, k1_valid, acc, h_used);
       else
         res = attempt_fp64<METRIC>(PL, R, K, k1_valid, acc, h_used);
       n_att += 1;
@@ -304,7 +378,7 @@ __global__ void __launch_bounds__(kTraceBlock,
             double c[8];
             cross_at(1, PL.max_radius, (PL.max_radius - xb[1]) / (raw[1] - xb[1]), c);
             if (OL.cross) {
-              store_cross(PL, OL, idx, c);
+              if (writer) store_cross(PL, OL, idx, c);
               crossed = true;
             }
             if (kSkyCross && PL.sky == kSkyChecker) {
@@ -332,7 +406,7 @@ __global__ void __launch_bounds__(kTraceBlock,
                 R.v[i] = c[4 + i];
               }
               R.lam = lam_b + s * h_used;
-              store_cross(PL, OL, idx, c);
+              if (writer) store_cross(PL, OL, idx, c);
               crossed = true;
               done_cls = kClsDisk;
             }
@@ -414,14 +488,17 @@ __global__ void __launch_bounds__(kTraceBlock,
         continue;
       }
       if (SCENE && done_cls == kClsScene) {
-        finish_scene_sample(PL, OL, idx, R, n_att, n_acc, inten, scene_rgb);
-        atomicAdd(&bs.attempts, (unsigned long long)n_att);
-        atomicAdd(&bs.accepted, (unsigned long long)n_acc);
-        atomicAdd(&bs.cls[kClsScene], 1ull);
+        if (writer) {
+          finish_scene_sample(PL, OL, idx, R, n_att, n_acc, inten, scene_rgb);
+          atomicAdd(&bs.attempts, (unsigned long long)n_att);
+          atomicAdd(&bs.accepted, (unsigned long long)n_acc);
+          atomicAdd(&bs.cls[kClsScene], 1ull);
+        }
         budget_pending += n_att;
         live = false;
       } else if (done_cls >= 0) {
-        finish(PL, OL, idx, done_cls, R, n_att, n_acc, out_int, out_temp, crossed,
+        if (writer)
+          finish(PL, OL, idx, done_cls, R, n_att, n_acc, out_int, out_temp, crossed,
                sky_at_cross ? sky_th : R.x[2], sky_at_cross ? sky_ph : R.x[3]);
         if (CKPT) O.diff_rays[idx] = DiffRay{n_acc, n_ckpt, done_cls, 0u};
         if (SRC == kSrcQueue) atomicAdd(&bs.fp64_att, (unsigned long long)(n_att - n_att0));
@@ -482,10 +559,44 @@ __global__ void reduce_samples_kernel(const __grid_constant__ DevParams P, const
 }
 
 template <int METRIC, int DISK, int STEPPER, int SRC, bool BATCH = false, bool SCENE = false,
-          bool CKPT = false, bool SMALL = false>
+          bool CKPT = false, bool SMALL = false, bool GROUP = false>
 const void* trace_fn() {
   return reinterpret_cast<const void*>(
-      &trace_fp64_kernel<METRIC, DISK, STEPPER, SRC, BATCH, SCENE, CKPT, SMALL>);
+      &trace_fp64_kernel<METRIC, DISK, STEPPER, SRC, BATCH, SCENE, CKPT, SMALL, GROUP>);
+}
+
+template <int METRIC, int DISK, bool SCENE = false>
+const void* group_fn() {
+  return trace_fn<METRIC, DISK, kStepperReference, kSrcCamera, false, SCENE, false, false, true>();
+}
+
+// The group kernel of a render with the reference's step.
+template <int METRIC>
+const void* select_group_metric(const DevParams& P) {
+  if (P.scene)
+    return P.disk == kDiskVolumetric ? group_fn<METRIC, kDiskVolumetric, true>()
+                                     : group_fn<METRIC, kDiskNone, true>();
+  return P.disk == kDiskThin         ? group_fn<METRIC, kDiskThin>()
+         : P.disk == kDiskVolumetric ? group_fn<METRIC, kDiskVolumetric>()
+                                     : group_fn<METRIC, kDiskNone>();
+}
+
+const void* select_group(const DevParams& P) {
+  return P.metric == kMetricKerr ? select_group_metric<kMetricKerr>(P)
+                                 : select_group_metric<kMetricSchwarzschild>(P);
+}
+
+// Renders of so few samples are traced by the group kernel from the camera:
+// there each lane of the other kernel has at most one ray, and the time is one ray's
+// chain.  Lane per ray / group, ms: Schwarzschild with a thin disk at 32x24
+// 0.97 / 0.48, 128^2 1.53 / 1.02, 160^2 1.56 / 1.43, 200^2 1.93 / 1.88, 256^2
+// 1.92 / 2.76; Kerr without a disk at 64^2 1.96 / 1.36, 160^2 3.67 / 3.44, 200^2
+// 3.67 / 4.08.  So the line is at 2^15 samples.
+#ifndef GG_GROUP_MAX_RAYS
+#define GG_GROUP_MAX_RAYS 32768
+#endif
+bool group_render(const DevParams& P) {
+  return P.stepper == kStepperReference && !P.attempt_budget && P.n_rays <= GG_GROUP_MAX_RAYS;
 }
 
 // Kerr camera passes of fewer samples than this run the 4-CTA budget of the
@@ -535,6 +646,7 @@ const void* select_metric_disk(const DevParams& P) {
 }
 
 const void* select_trace(const DevParams& P) {
+  if (group_render(P)) return select_group(P);
   // gg_forward_ckpt admits only Kerr, the thin disk and the full stepper
   if (P.ckpt)
     return trace_fn<kMetricKerr, kDiskThin, kStepperDP45, kSrcCamera, false, false, true>();
@@ -568,6 +680,33 @@ cudaError_t trace_occupancy(const DevParams& P, int* blocks_per_sm) {
 cudaError_t queue_trace_occupancy(const DevParams& P, int* blocks_per_sm) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
       blocks_per_sm, select_queue_trace(P, false), kTraceBlock, 0);
+}
+
+int chain_capacity(const DevParams& P, int grid) {
+  if (P.stepper != kStepperReference || P.attempt_budget || group_render(P)) return 0;
+  return grid * (kTraceBlock / 32) * (int)kHandLanes;
+}
+
+uint64_t trace_blocks(const DevParams& P) {
+  const uint64_t per = group_render(P) ? kTraceBlock / kGroupLanes : kTraceBlock;
+  return (P.n_rays + per - 1) / per;
+}
+
+cudaError_t launch_group(const DevParams& P, const DevOutputs& O, DevControl* ctl, int sms,
+                         cudaStream_t stream) {
+  const void* fn = select_group(P);
+  int bps = 0;
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, kTraceBlock, 0);
+  if (e != cudaSuccess) return e;
+  // a CTA takes 128 / kGroupLanes rays at a time
+  const int most = (int)(O.chain_cap / (kTraceBlock / kGroupLanes)) + 1;
+  int grid = sms * (bps > 0 ? bps : 1);
+  if (grid > most) grid = most;
+  DevParams p = P;
+  DevOutputs o = O;
+  BatchTable b{};
+  void* args[] = {&p, &o, &ctl, &b};
+  return cudaLaunchKernel(fn, dim3(grid), dim3(kTraceBlock), args, 0, stream);
 }
 
 cudaError_t launch_queue_trace(const DevParams& P, const DevOutputs& O, DevControl* ctl,
