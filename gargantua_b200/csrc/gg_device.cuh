@@ -54,11 +54,17 @@ struct KerrGeo {
   T hrr, hthth;        // -g^rr / 2, -g^thth / 2
 };
 
-// 1/x: IEEE division in FP64; in the mixed form's FP32 right-hand side the
-// fast reciprocal (__fdividef, within 2 ulp), whose arguments there stay in
-// the normal range (r is outside the FP64 band, theta away from the poles).
+// 1/x: IEEE division in FP64; in the mixed form's FP32 right-hand side and
+// error scales the hardware reciprocal (within 1 ulp).  Its arguments there are normal numbers (r
+// is outside the FP64 band, theta away from the poles, a scale at least
+// FLT_MIN), for which __fdividef(1, x) gives the same bits after a range
+// test and two scalings.
 GG_DEV double rcp(double x) { return 1.0 / x; }
-GG_DEV float rcp(float x) { return __fdividef(1.0f, x); }
+GG_DEV float rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 
 template <class T>
 GG_DEV KerrGeo<T> kerr_geometry(T M, T a, T r, T s, T c) {

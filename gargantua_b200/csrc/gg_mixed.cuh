@@ -598,8 +598,8 @@ GG_DEV int attempt_dp45_mixed(const DevParams& P, MixedRegs& S, const KS& K,
     for (int i = 0; i < 4; ++i) {
       const float xs = fmaf(P.rtol_f, fmaxf(fabsf(xh[i]), fabsf(xh[i] + dx[i])), P.atol_f);
       const float vs = fmaf(P.rtol_f, fmaxf(fabsf(S.vh[i]), fabsf(S.vh[i] + dv[i])), P.atol_f);
-      const double qx = (hhd * ex[i]) * (double)__fdividef(1.0f, xs);
-      const double qv = (hd * ev[i]) * (double)__fdividef(1.0f, vs);
+      const double qx = (hhd * ex[i]) * (double)rcp(xs);
+      const double qv = (hd * ev[i]) * (double)rcp(vs);
       s2 = fma(qx, qx, fma(qv, qv, s2));
     }
 #if GG_MIXED_ROOT10
