@@ -1,5 +1,5 @@
-// gg_adjoint.cu -- the differentiable render: forward pass with checkpoints
-// and the hand-written adjoint (reverse-mode) pass.
+// gg_adjoint.cu -- the differentiable render: the hand-written adjoint
+// (reverse-mode) pass over the forward's checkpoints.
 //
 // Image: Kerr, thin disk, one sample per pixel, full Dormand-Prince stepper
 // in FP64.  Each pixel's linear colour is a function of five parameters:
@@ -14,23 +14,39 @@
 // gg_trace.cu), which also stores each ray's state (x, v, next h) at the start
 // and after every kCkptEvery-th accepted step, and its DiffRay.
 //
-// Backward (diff_backward_kernel), per disk ray, given dL/d(colour):
-//   1. the crossing step (the last accepted step) again in forward-mode dual
-//      numbers over its start state (8) and the spin: stages, continuous
-//      extension, the root s* (one Newton correction in dual arithmetic gives
-//      ds*/dp by the implicit function theorem), the crossing state, the
-//      redshift and I -- so dL/d(start state), dL/da, dL/dr_in, dL/dq and
-//      dL/d(observer normalisation) in one pass;
-//   2. every earlier step in reverse, segment by segment: the segment is
-//      replayed from its checkpoint (the controller is deterministic, so the
-//      replay takes the same steps), then the adjoint goes back through each
-//      step's Dormand-Prince stages (vector-Jacobian products of each
-//      stage's Kerr right-hand side in r, theta, the stage velocity and the
-//      spin, by a hand-written reverse pass, gg_vjp.cuh), with theta
-//      reflections at the poles reversing its adjoint;
-//   3. the camera: the initial state and the observer normalisation as
+// Backward, over the disk rays with a nonzero dL/d(colour), in five launches:
+//   1. a counting sort lists the rays by their number of segments, longest
+//      first (backward_count / backward_scatter; the host makes the prefix
+//      sums in between);
+//   2. backward_replay_kernel: every segment of every listed ray is replayed
+//      from its checkpoint, a lane each (the controller is deterministic, so a
+//      replay takes the forward's steps), and leaves each step's start, size and
+//      stage derivatives in a record;
+//   3. backward_crossing_kernel: the crossing step (a ray's last) again in
+//      forward-mode dual numbers over its start state (6) and the spin: stages,
+//      continuous extension, the root s* (one Newton correction in dual
+//      arithmetic gives ds*/dp by the implicit function theorem), the crossing
+//      state, the redshift and I -- so dL/d(start state), dL/da, dL/dr_in,
+//      dL/dq and dL/d(observer normalisation) in one pass;
+//   4. backward_chain_kernel: the steps before it in reverse, each the
+//      vector-Jacobian products of its stages' Kerr right-hand sides in r, theta,
+//      the stage velocity and the spin, by a hand-written reverse pass
+//      (gg_vjp.cuh), with theta reflections at the poles reversing its adjoint.
+//      A lane takes a ray's last few segments one after the other;
+//      of a longer ray, each earlier segment is taken by six lanes, one per
+//      component of the adjoint, at the same time: they give the segment's
+//      transposed Jacobian;
+//   5. backward_camera_kernel: the long rays' adjoints through those Jacobians,
+//      then the camera: the initial state and the observer normalisation as
 //      3-direction duals in (a, inclination, r_cam), contracted with the
-//      adjoint of the initial state.
+//      adjoint of the initial state, and the five sums.
+// The adjoint of t and phi is zero throughout (neither the metric nor the colour
+// depends on them), so six components are carried.  What bounds it: one ray's
+// chain.  Replayed and taken back by one lane, the longest ray of the 512^2
+// image (673 steps, the median being 39) took 8.6 ms, its warp issuing every
+// fourth cycle.  With the segments in parallel the longest chain is 32 to 128
+// steps, and the launches of the 512^2 backward take 0.9 (replay), 0.6 (crossing)
+// and 1.5 ms (chain): 9.2 ms before, 3.0 after; 128^2 2.95 / 0.72 ms.
 // The step sizes are held fixed (the adjoint of the discrete map with the
 // forward's accepted steps; their own dependence on the parameters moves the
 // solution by the truncation error only).
@@ -43,26 +59,6 @@
 #include "gg_vjp.cuh"
 #include "gg_launch.h"
 #include "gg_trace_common.cuh"
-
-// Build knobs of the backward (tuning builds compare them).  GG_ADJ_HAND_VJP:
-// each stage's vector-Jacobian product by the hand-written reverse pass
-// (kerr_rhs_vjp_hand) instead of dual numbers.  GG_ADJ_STORE_K: the replay
-// keeps each accepted step's stage derivatives for the step's product instead
-// of evaluating them again.  GG_ADJ_MIN_BLOCKS: the CTAs per SM the backward's
-// registers are budgeted for (1 leaves the compiler's own choice).  Measured
-// on the 512^2 gradient (backward ms): dual numbers 11.2, dual with kept stages
-// 9.9, hand-written 8.5, hand-written with kept stages 7.9 (the default; the
-// forward takes 8.8); the gradients agree to 1e-15.  The same at 3 CTAs per SM
-// (168 registers, twice the spill code): 9.0.
-#ifndef GG_ADJ_HAND_VJP
-#define GG_ADJ_HAND_VJP 1
-#endif
-#ifndef GG_ADJ_STORE_K
-#define GG_ADJ_STORE_K 1
-#endif
-#ifndef GG_ADJ_MIN_BLOCKS
-#define GG_ADJ_MIN_BLOCKS 1
-#endif
 
 namespace gg {
 
@@ -98,103 +94,150 @@ GG_DEV T redshift_eq(double M, const T& a, const T& r, const T v[4]) {
 }
 
 // ---- backward -----------------------------------------------------------------
+// Threads per CTA of the chain kernel and CTAs per SM: 255 registers, which
+// still spill a little; at 168 (5 or 6 CTAs) the 512^2 backward took 3.7 ms
+// instead of 3.4.
+constexpr int kChainBlock = 64, kChainMinBlocks = 4;
+constexpr int kRecDoubles = 31;   // a step's record: r, theta, v, h, k_1 .. k_6
+// Records of 32 items side by side, so that a warp's accesses are coalesced:
+// value c of step j of item i.
+GG_DEV uint64_t rec_at(uint64_t i, uint32_t j, int c) {
+  return ((i / 32) * (kCkptEvery * kRecDoubles) + j * kRecDoubles + c) * 32 + i % 32;
+}
+
+// This thread's columns of the chain kernel's shared memory: a step's stage
+// derivatives and its stages' products (Xr, Xth, W).
+struct ChainStore {
+  double2 (*k)[2][kChainBlock];  // [6]
+  double2 (*x)[3][kChainBlock];  // [6]
+  GG_DEV void get_k(int l, double out[4]) const {
+    const double2 a = k[l][0][threadIdx.x], b = k[l][1][threadIdx.x];
+    out[0] = a.x;
+    out[1] = a.y;
+    out[2] = b.x;
+    out[3] = b.y;
+  }
+  GG_DEV void set_k(int l, const double in[4]) const {
+    k[l][0][threadIdx.x] = make_double2(in[0], in[1]);
+    k[l][1][threadIdx.x] = make_double2(in[2], in[3]);
+  }
+  GG_DEV void get_x(int s, double out[6]) const {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const double2 a = x[s][j][threadIdx.x];
+      out[2 * j] = a.x;
+      out[2 * j + 1] = a.y;
+    }
+  }
+  GG_DEV void set_x(int s, const double in[6]) const {
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      x[s][j][threadIdx.x] = make_double2(in[2 * j], in[2 * j + 1]);
+  }
+};
+
+// Stage S's r, theta and velocity, and its cotangent kb = dL/dk_S from the
+// step's outputs and the later stages' products.
+template <int S>
+GG_DEV void vjp_stage(const ChainStore& C, double r, double th, const double v[4], double h,
+                      double hh, const double lx[2], const double lv[4], double& pr, double& pth,
+                      double w[4], double kb[4]) {
+  const double ha = h * kDP.A[S];
+  pr = fma(ha, v[1], r);
+  pth = fma(ha, v[2], th);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) w[i] = v[i];
+#pragma unroll
+  for (int l = 0; l < S; ++l) {
+    double k[4];
+    C.get_k(l, k);
+    const double cv = h * kDP.B[S][l];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = fma(cv, k[i], w[i]);
+    if (l < S - 1) {
+      const double cb = hh * kDP.Abar[S][l];
+      pr = fma(cb, k[1], pr);
+      pth = fma(cb, k[2], pth);
+    }
+  }
+  const double cb6 = hh * kDP.Abar[6][S], cv6 = h * kDP.B[6][S];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) kb[i] = cv6 * lv[i];
+  kb[1] = fma(cb6, lx[0], kb[1]);
+  kb[2] = fma(cb6, lx[1], kb[2]);
+#pragma unroll
+  for (int j = S + 1; j < 6; ++j) {
+    double x[6];
+    C.get_x(j, x);
+    const double cb = hh * kDP.Abar[j][S], cv = h * kDP.B[j][S];
+    kb[0] = fma(cv, x[2], kb[0]);
+    kb[1] = fma(cb, x[0], fma(cv, x[3], kb[1]));
+    kb[2] = fma(cb, x[1], fma(cv, x[4], kb[2]));
+    kb[3] = fma(cv, x[5], kb[3]);
+  }
+}
+
 // Vector-Jacobian product through one accepted full Dormand-Prince step
-// (Nystrom form, attempt_dp45_fp64): (lx, lv) is dL/d(x_new, v_new) on entry
-// and dL/d(x, v) on return; dL/da is accumulated into *ga.
-// kst: the step's stage derivatives k_1..k_6 as the forward took them, or
-// null to evaluate them again here.
-GG_DEV void dp45_vjp(const DevParams& P, const double x[4], const double v[4], double h,
-                     const double (*kst)[4], double lx[4], double lv[4], double* ga) {
-  double k[6][4], pr[6], pth[6], pw[6][4];
+// (Nystrom form, attempt_dp45_fp64), its stage derivatives in C: (lx, lv) is
+// dL/d(r, theta, v) at its end on entry and at its start on return; dL/da is
+// accumulated into *ga.
+GG_DEV void step_vjp(const DevParams& P, const ChainStore& C, double r, double th,
+                     const double v[4], double h, double lx[2], double lv[4], double* ga) {
   const double hh = h * h;
-  for (int s = 0; s < 6; ++s) {
-    double px[4], w[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      px[i] = fma(h * kDP.A[s], v[i], x[i]);
-      w[i] = v[i];
-    }
-    for (int l = 0; l < s; ++l)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        px[i] = fma(hh * kDP.Abar[s][l], k[l][i], px[i]);
-        w[i] = fma(h * kDP.B[s][l], k[l][i], w[i]);
-      }
-    if (kst) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) k[s][i] = kst[s][i];
-    } else {
-      Geometry<kMetricKerr, kStepperDP45> G;
-      G.at(P, px[1], px[2]);
-      G.accel(w, k[s]);
-    }
-    pr[s] = px[1];
-    pth[s] = px[2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) pw[s][i] = w[i];
-  }
-  double kb[6][4];
-  for (int l = 0; l < 6; ++l)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) kb[l][i] = 0.0;
-  // outputs: x_new = x + h v + h^2 sum Abar[6][l] k_l, v_new = v + h sum B[6][l] k_l
-  double xbar[4], vbar[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    xbar[i] = lx[i];
-    vbar[i] = lv[i] + h * lx[i];
-  }
-  for (int l = 0; l < 6; ++l)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) kb[l][i] += hh * kDP.Abar[6][l] * lx[i] + h * kDP.B[6][l] * lv[i];
+  // x_new = x + h v + ..., v_new = v + ...
+  double xb[2] = {lx[0], lx[1]};
+  double vb[4] = {lv[0], fma(h, lx[0], lv[1]), fma(h, lx[1], lv[2]), lv[3]};
+#pragma unroll 1
   for (int s = 5; s >= 0; --s) {
-    // k_s = f(r_s, theta_s, w_s; a), back through its Jacobian
-    double Xr = 0.0, Xth = 0.0, W[4] = {0.0, 0.0, 0.0, 0.0};
-#if GG_ADJ_HAND_VJP
-    kerr_rhs_vjp_hand(P.mass, P.spin, pr[s], pth[s], pw[s], kb[s], &Xr, &Xth, W, ga);
-#else
-    kerr_rhs_vjp_dual(P.mass, P.spin, pr[s], pth[s], pw[s], kb[s], &Xr, &Xth, W, ga);
-#endif
-    // x_s = x + h A_s v + h^2 sum_{l<s} Abar k_l ; w_s = v + h sum_{l<s} B k_l
-    xbar[1] += Xr;
-    xbar[2] += Xth;
-    vbar[1] += h * kDP.A[s] * Xr;
-    vbar[2] += h * kDP.A[s] * Xth;
-#pragma unroll
-    for (int m = 0; m < 4; ++m) vbar[m] += W[m];
-    for (int l = 0; l < s; ++l) {
-      const double cb = hh * kDP.Abar[s][l], cv = h * kDP.B[s][l];
-      kb[l][1] += cb * Xr;
-      kb[l][2] += cb * Xth;
-#pragma unroll
-      for (int m = 0; m < 4; ++m) kb[l][m] += cv * W[m];
+    double pr, pth, w[4], kb[4];
+    switch (s) {
+      case 0: vjp_stage<0>(C, r, th, v, h, hh, lx, lv, pr, pth, w, kb); break;
+      case 1: vjp_stage<1>(C, r, th, v, h, hh, lx, lv, pr, pth, w, kb); break;
+      case 2: vjp_stage<2>(C, r, th, v, h, hh, lx, lv, pr, pth, w, kb); break;
+      case 3: vjp_stage<3>(C, r, th, v, h, hh, lx, lv, pr, pth, w, kb); break;
+      case 4: vjp_stage<4>(C, r, th, v, h, hh, lx, lv, pr, pth, w, kb); break;
+      default: vjp_stage<5>(C, r, th, v, h, hh, lx, lv, pr, pth, w, kb); break;
     }
+    // k_s = f(r_s, theta_s, w_s; a), back through its Jacobian
+    double x[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    kerr_rhs_vjp_hand(P.mass, P.spin, pr, pth, w, kb, &x[0], &x[1], &x[2], ga);
+    if (s > 0) C.set_x(s, x);
+    // r_s = r + h A_s v_r + ..., w_s = v + ...
+    const double ha = h * kDP.A[s];
+    xb[0] += x[0];
+    xb[1] += x[1];
+    vb[0] += x[2];
+    vb[1] += fma(ha, x[0], x[3]);
+    vb[2] += fma(ha, x[1], x[4]);
+    vb[3] += x[5];
   }
+  lx[0] = xb[0];
+  lx[1] = xb[1];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    lx[i] = xbar[i];
-    lv[i] = vbar[i];
-  }
+  for (int i = 0; i < 4; ++i) lv[i] = vb[i];
 }
 
 // dL/d(start state of the crossing step) and the parameter terms of the
 // crossing: the step, its continuous extension and root, the redshift and the
-// disk colour in 9-direction duals (8 state components, spin).  dl: dL/d rgb.
+// disk colour in 7-direction duals (r, theta, the velocity, the spin;
+// nothing depends on t and phi).  dl: dL/d rgb.
 // Returns false when the step does not reach the disk (no contribution).
 GG_DEV bool crossing_vjp(const DevParams& P, const double xb[4], const double vb[4], double h,
-                         const double dl[3], double lam[8], double* ga, double* g_rin,
+                         const double dl[3], double lam[6], double* ga, double* g_rin,
                          double* g_q, double* g_sobs) {
-  using D9 = Dual<9>;
-  D9 x[4], v[4], k[7][4], xa[4], va[4];
+  using D7 = Dual<7>;
+  D7 x[4], v[4], k[7][4], xa[4], va[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    x[i] = D9::var(xb[i], i);
-    v[i] = D9::var(vb[i], 4 + i);
+    x[i] = D7(xb[i]);
+    v[i] = D7::var(vb[i], 2 + i);
   }
-  const D9 a = D9::var(P.spin, 8);
+  x[1].d[0] = 1.0;
+  x[2].d[1] = 1.0;
+  const D7 a = D7::var(P.spin, 6);
   const double hh = h * h;
   for (int s = 0; s < 7; ++s) {
-    D9 px[4], w[4];
+    D7 px[4], w[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       px[i] = x[i] + (h * kDP.A[s]) * v[i];
@@ -206,7 +249,7 @@ GG_DEV bool crossing_vjp(const DevParams& P, const double xb[4], const double vb
         px[i] = px[i] + (hh * kDP.Abar[s][l]) * k[l][i];
         w[i] = w[i] + (h * kDP.B[s][l]) * k[l][i];
       }
-    kerr_rhs_dual<9>(P.mass, a, px[1], px[2], w, k[s]);
+    kerr_rhs_dual<7>(P.mass, a, px[1], px[2], w, k[s]);
     if (s == 6) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -216,10 +259,10 @@ GG_DEV bool crossing_vjp(const DevParams& P, const double xb[4], const double vb
     }
   }
   // continuous extension coefficients of the 8 components
-  D9 y0[8], r2[8], r3[8], r4[8], r5[8];
+  D7 y0[8], r2[8], r3[8], r4[8], r5[8];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    D9 sx(0.0), sv(0.0);
+    D7 sx(0.0), sv(0.0);
     for (int l = 0; l < 7; ++l) {
       sx = sx + kDP.Dbar[l] * k[l][i];
       sv = sv + kDP.D[l] * k[l][i];
@@ -250,17 +293,17 @@ GG_DEV bool crossing_vjp(const DevParams& P, const double xb[4], const double vb
   sp.h = h;
   double cval[8];
   const double s0 = dense_crossing(sp, 2, kHalfPi, cval);
-  auto poly = [&](int c, const D9& s) {
-    const D9 t = 1.0 - s;
+  auto poly = [&](int c, const D7& s) {
+    const D7 t = 1.0 - s;
     return y0[c] + s * (r2[c] + t * (r3[c] + s * (r4[c] + t * r5[c])));
   };
-  const D9 sd0(s0);
-  const D9 f = poly(2, sd0) - kHalfPi;
+  const D7 sd0(s0);
+  const D7 f = poly(2, sd0) - kHalfPi;
   const double t0 = 1.0 - s0;
   const double fp = r2[2].v + (1.0 - 2.0 * s0) * r3[2].v + s0 * (2.0 - 3.0 * s0) * r4[2].v +
                     2.0 * s0 * t0 * (1.0 - 2.0 * s0) * r5[2].v;
-  const D9 sd = sd0 - f / fp;
-  const D9 rc = poly(1, sd);
+  const D7 sd = sd0 - f / fp;
+  const D7 rc = poly(1, sd);
   double rcv = rc.v;
   {
     double cn[8];
@@ -270,22 +313,22 @@ GG_DEV bool crossing_vjp(const DevParams& P, const double xb[4], const double vb
     rcv = cn[1];
   }
   if (!(rcv >= P.r_inner && rcv <= P.r_outer)) return false;
-  D9 vc[4];
+  D7 vc[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) vc[i] = poly(4 + i, sd);
   // g (observer normalisation s_obs factored out), I = g^4 (r_in / r_c)^q
-  const D9 g0 = redshift_eq<D9>(P.mass, a, rc, vc);
-  const D9 g = g0 / P.sqrt_neg_gtt_obs;
-  const D9 g2 = g * g;
-  const D9 I = (g2 * g2) * pow(P.r_inner / rc, P.emissivity_index);
+  const D7 g0 = redshift_eq<D7>(P.mass, a, rc, vc);
+  const D7 g = g0 / P.sqrt_neg_gtt_obs;
+  const D7 g2 = g * g;
+  const D7 I = (g2 * g2) * pow(P.r_inner / rc, P.emissivity_index);
   // dL/dI through the disk colour (x^0.5, x^1.2, x^2.5), x = I / (1 + I)
   const double xv = I.v / (1.0 + I.v);
   const double dx = 1.0 / ((1.0 + I.v) * (1.0 + I.v));
   const double dLdI = dx * (dl[0] * 0.5 * ::pow(xv, -0.5) + dl[1] * 1.2 * ::pow(xv, 0.2) +
                             dl[2] * 2.5 * ::pow(xv, 1.5));
 #pragma unroll
-  for (int j = 0; j < 8; ++j) lam[j] = dLdI * I.d[j];
-  *ga += dLdI * I.d[8];
+  for (int j = 0; j < 6; ++j) lam[j] = dLdI * I.d[j];
+  *ga += dLdI * I.d[6];
   *g_rin += dLdI * I.v * P.emissivity_index / P.r_inner;
   *g_q += dLdI * I.v * ::log(P.r_inner / rc.v);
   *g_sobs += dLdI * (-4.0 * I.v / P.sqrt_neg_gtt_obs);
@@ -340,124 +383,53 @@ GG_DEV void camera_dual(const DevParams& P, double u, double v, Dual<3> y0[8], D
   *sobs = sqrt(-gtt);
 }
 
-// Replays one segment of accepted steps from a checkpoint, recording each
-// step's start state, size and whether its end was reflected at a pole, and
-// (Kst non-null) its stage derivatives k_1..k_6.
-GG_DEV void replay(const DevParams& P, const Ckpt& c0, uint32_t steps, double S[][8], double* H,
-                   double (*Kst)[6][4], uint32_t* refl) {
-  double kl[7][4];
-  const KStoreLocal K{kl};
-  Ray R;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    R.x[i] = c0.x[i];
-    R.v[i] = c0.v[i];
-  }
-  R.h = c0.h;
-  R.lam = 0.0;
-  bool k1v = false, k7p = false;
-  *refl = 0u;
-  for (uint32_t j = 0; j < steps; ++j) {
-    for (uint32_t guard = 0; guard < 100000u; ++guard) {
-      double xb[4], vb[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        xb[i] = R.x[i];
-        vb[i] = R.v[i];
-      }
-      bool acc;
-      double h_used = 0.0;
-      StepEnd end;
-      attempt_dp45_fp64<kMetricKerr>(P, R, K, k1v, k7p, acc, h_used, end);
-      if (acc) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          S[j][i] = xb[i];
-          S[j][4 + i] = vb[i];
-        }
-        H[j] = h_used;
-        if (Kst)
-          for (int l = 0; l < 6; ++l)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) Kst[j][l][i] = kl[l][i];
-        if (end.xraw[2] < 0.0 || end.xraw[2] > kPi) *refl |= 1u << j;
-        break;
-      }
-    }
-  }
-}
-
-// The adjoint of one disk ray (sample idx) given dL/d(colour), its five
-// sums added to acc5.
-GG_DEV void backward_ray(const DevParams& P, const DiffOut& D, const double* dl_drgb,
-                         uint64_t idx, double acc5[5]) {
-  const DiffRay dr = D.rays[idx];
-  if (dr.cls != kClsDisk || dr.n_acc == 0) return;
-  const double dl[3] = {dl_drgb[3 * idx], dl_drgb[3 * idx + 1], dl_drgb[3 * idx + 2]};
-  if (dl[0] == 0.0 && dl[1] == 0.0 && dl[2] == 0.0) return;
-  const uint32_t n_ck = dr.n_ckpt < D.ckpt_per_ray ? dr.n_ckpt : D.ckpt_per_ray;
-  const Ckpt* ck = D.ckpt + idx * D.ckpt_per_ray;
-  double lam[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  double ga = 0.0, g_rin = 0.0, g_q = 0.0, g_sobs = 0.0;
-  double S[kCkptEvery][8], H[kCkptEvery];
-#if GG_ADJ_STORE_K
-  double Kst[kCkptEvery][6][4];
-#else
-  double (*Kst)[6][4] = nullptr;
-#endif
-  bool ok = true;
-  for (int seg = (int)n_ck - 1; seg >= 0 && ok; --seg) {
-    const uint32_t first = (uint32_t)seg * kCkptEvery;
-    const uint32_t steps = seg == (int)n_ck - 1 ? dr.n_acc - first : (uint32_t)kCkptEvery;
-    if (steps == 0 || steps > (uint32_t)kCkptEvery) {
-      ok = false;
-      break;
-    }
-    uint32_t refl = 0;
-    replay(P, ck[seg], steps, S, H, Kst, &refl);
-    for (int j = (int)steps - 1; j >= 0; --j) {
-      if (seg == (int)n_ck - 1 && j == (int)steps - 1) {
-        ok = crossing_vjp(P, S[j], S[j] + 4, H[j], dl, lam, &ga, &g_rin, &g_q, &g_sobs);
-        if (!ok) break;
-        continue;
-      }
-      if (refl & (1u << j)) lam[2] = -lam[2];  // theta -> -theta or 2 pi - theta
-      dp45_vjp(P, S[j], S[j] + 4, H[j], Kst ? Kst[j] : nullptr, lam, lam + 4, &ga);
-    }
-  }
-  if (!ok) return;
-  double u, v;
-  sample_uv(P, idx, u, v);
-  Dual<3> y0[8], sobs;
-  camera_dual(P, u, v, y0, &sobs);
-  double g3[3] = {ga, 0.0, 0.0};
-#pragma unroll
-  for (int p = 0; p < 3; ++p) {
-    for (int j = 0; j < 8; ++j) g3[p] += lam[j] * y0[j].d[p];
-    g3[p] += g_sobs * sobs.d[p];
-  }
-  acc5[0] += g3[0];
-  acc5[1] += g3[1];
-  acc5[2] += g3[2];
-  acc5[3] += g_rin;
-  acc5[4] += g_q;
-}
-
-// Work list of the backward pass: the disk rays with a nonzero dL/d(colour),
-// longest first, by a counting sort on the checkpoint count (segments of
-// kCkptEvery accepted steps).  Warps claim 32 rays of about equal length at a
-// time (on the 512^2 image the lanes' useful share of a warp's steps goes from
-// 0.78 to 1.0), and the longest chains, which set the pass's tail, start at
-// once instead of in a later wave of blocks.
-struct BackwardList {
-  unsigned long long* head;  // next entry to claim
-  uint32_t* total;           // entries in the list
-  uint32_t* bins;            // per key: its count, then (after the scan) its next slot
-  uint64_t* list;            // sample indices
-  uint32_t n_keys;           // = D.ckpt_per_ray
+// ---- the work list ---------------------------------------------------------------
+// Listed rays of the same number of segments: the first one's place in the
+// list, and the segments ("items") and parallel segments of all rays before it.
+struct BackwardBin {
+  uint64_t start, item, par;
+  uint32_t segs, pad;
 };
 
-constexpr int kScanThreads = 1024;
+// A window of the list: entries [e0, e1) with items from g0 and parallel
+// segments from p0, and where the kernels leave their results.
+struct BackwardWork {
+  const uint64_t* list;      // sample indices
+  const BackwardBin* bins;   // n_bins, and one past the end with the totals
+  uint32_t n_bins;
+  uint32_t tail;  // segments of a ray that one lane takes in sequence
+  uint64_t e0, e1, g0, g1, p0, p1;
+  double* rec;  // step records of the window's items
+  double* ray;  // [kRayDoubles][e1 - e0]
+  double* par;  // [p1 - p0][6][7]
+};
+constexpr int kRayDoubles = 11;  // dL/d(r, theta, v), dL/da, dL/dr_in, dL/dq, dL/ds_obs, valid
+
+struct BackwardEntry {
+  uint64_t e, item, par;  // place in the list, its first item and parallel segment
+  uint32_t segs;
+};
+
+GG_DEV uint32_t parallel_segments(const BackwardWork& W, uint32_t segs) {
+  return segs > W.tail ? segs - W.tail : 0u;
+}
+
+// The last bin whose `field` is at most `at`.
+template <uint64_t BackwardBin::*FIELD>
+GG_DEV uint32_t find_bin(const BackwardWork& W, uint64_t at) {
+  uint32_t lo = 0, hi = W.n_bins;
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (W.bins[mid].*FIELD <= at) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+GG_DEV BackwardEntry entry_at(const BackwardWork& W, uint64_t e) {
+  const BackwardBin& b = W.bins[find_bin<&BackwardBin::start>(W, e)];
+  const uint64_t k = e - b.start;
+  return {e, b.item + k * b.segs, b.par + k * parallel_segments(W, b.segs), b.segs};
+}
 
 GG_DEV bool backward_key(const DiffOut& D, const double* dl, uint64_t idx, uint32_t* key) {
   const DiffRay dr = D.rays[idx];
@@ -469,13 +441,21 @@ GG_DEV bool backward_key(const DiffOut& D, const double* dl, uint64_t idx, uint3
   return true;
 }
 
+// Steps of segment `seg` of a ray with n_acc accepted ones; 0 if the counts do
+// not fit together (the ray then has no gradient).
+GG_DEV uint32_t segment_steps(uint32_t n_acc, uint32_t segs, uint32_t seg) {
+  if (seg + 1 < segs) return (uint32_t)kCkptEvery;
+  const uint32_t first = seg * kCkptEvery;
+  return n_acc > first && n_acc - first <= (uint32_t)kCkptEvery ? n_acc - first : 0u;
+}
+
 // Neighbouring disk rays mostly share a key: the lanes of a warp with the
 // same key take their slots with one atomic (count and scatter), which keeps
 // the popular bins from serialising.  The loops run the same trips on every
 // lane of a block, so the warp-wide votes see all 32 lanes.
 __global__ void backward_count_kernel(const __grid_constant__ DevParams P,
                                       const __grid_constant__ DiffOut D, const double* dl,
-                                      BackwardList L) {
+                                      uint32_t* bins) {
   const unsigned lane = threadIdx.x & 31u;
   for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < P.n_rays;
        base += (uint64_t)gridDim.x * blockDim.x) {
@@ -483,40 +463,14 @@ __global__ void backward_count_kernel(const __grid_constant__ DevParams P,
     uint32_t k = 0;
     const bool has = idx < P.n_rays && backward_key(D, dl, idx, &k);
     const unsigned grp = __match_any_sync(kFull, has ? k : 0xffffffffu);
-    if (has && lane == (unsigned)(__ffs(grp) - 1)) atomicAdd(L.bins + k, (uint32_t)__popc(grp));
+    if (has && lane == (unsigned)(__ffs(grp) - 1)) atomicAdd(bins + k, (uint32_t)__popc(grp));
   }
 }
 
-// Exclusive prefix sum of the key counts, in place, and the total (one block
-// of kScanThreads threads, each over a contiguous run of keys).
-__global__ void __launch_bounds__(kScanThreads) backward_scan_kernel(BackwardList L) {
-  __shared__ uint32_t part[kScanThreads];
-  const uint32_t t = threadIdx.x;
-  const uint32_t per = (L.n_keys + kScanThreads - 1) / kScanThreads;
-  const uint32_t b0 = t * per < L.n_keys ? t * per : L.n_keys;
-  const uint32_t b1 = b0 + per < L.n_keys ? b0 + per : L.n_keys;
-  uint32_t sum = 0;
-  for (uint32_t b = b0; b < b1; ++b) sum += L.bins[b];
-  part[t] = sum;
-  __syncthreads();
-  for (uint32_t off = 1; off < kScanThreads; off <<= 1) {
-    const uint32_t v = t >= off ? part[t - off] : 0u;
-    __syncthreads();
-    part[t] += v;
-    __syncthreads();
-  }
-  uint32_t run = t ? part[t - 1] : 0u;
-  for (uint32_t b = b0; b < b1; ++b) {
-    const uint32_t c = L.bins[b];
-    L.bins[b] = run;
-    run += c;
-  }
-  if (t == kScanThreads - 1) *L.total = part[t];
-}
-
+// `next`: per key, the next free place of the list.
 __global__ void backward_scatter_kernel(const __grid_constant__ DevParams P,
                                         const __grid_constant__ DiffOut D, const double* dl,
-                                        BackwardList L) {
+                                        unsigned long long* next, uint64_t* list) {
   const unsigned lane = threadIdx.x & 31u;
   for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < P.n_rays;
        base += (uint64_t)gridDim.x * blockDim.x) {
@@ -526,28 +480,210 @@ __global__ void backward_scatter_kernel(const __grid_constant__ DevParams P,
     const unsigned grp = __match_any_sync(kFull, has ? k : 0xffffffffu);
     if (has) {
       const unsigned leader = (unsigned)(__ffs(grp) - 1);
-      uint32_t first = 0;
-      if (lane == leader) first = atomicAdd(L.bins + k, (uint32_t)__popc(grp));
+      unsigned long long first = 0;
+      if (lane == leader) first = atomicAdd(next + k, (unsigned long long)__popc(grp));
       first = __shfl_sync(grp, first, leader);
-      L.list[first + (uint32_t)__popc(grp & lanemask_lt())] = idx;
+      list[first + (uint32_t)__popc(grp & lanemask_lt())] = idx;
     }
   }
 }
 
-// Persistent: each warp claims the next 32 entries of the sorted list.
-__global__ void __launch_bounds__(128, GG_ADJ_MIN_BLOCKS) diff_backward_kernel(const __grid_constant__ DevParams P,
-                                                            const __grid_constant__ DiffOut D,
-                                                            const double* dl_drgb,
-                                                            double* grad5, BackwardList L) {
+// Replays the window's segments, a lane each, and records their steps (the
+// size negated where the step's end was reflected at a pole).
+__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocksKerrChain)
+    backward_replay_kernel(const __grid_constant__ DevParams P, const __grid_constant__ DiffOut D,
+                           const __grid_constant__ BackwardWork W) {
+  __shared__ double2 k_smem[7][2][kTraceBlock];
+  const KStore K{k_smem};
+  const uint64_t g = W.g0 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= W.g1) return;
+  const BackwardBin& b = W.bins[find_bin<&BackwardBin::item>(W, g)];
+  const uint64_t in_bin = g - b.item;
+  const uint32_t seg = (uint32_t)(in_bin % b.segs);
+  const uint64_t idx = W.list[b.start + in_bin / b.segs];
+  const uint32_t steps = segment_steps(D.rays[idx].n_acc, b.segs, seg);
+  const Ckpt& c0 = D.ckpt[idx * D.ckpt_per_ray + seg];
+  Ray R;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    R.x[i] = c0.x[i];
+    R.v[i] = c0.v[i];
+  }
+  R.h = c0.h;
+  R.lam = 0.0;
+  bool k1v = false, k7p = false;
+  double* const rec = W.rec + rec_at(g - W.g0, 0, 0);
+  uint32_t j = 0, tries = 0;
+  while (j < steps && tries < 100000u) {
+    double q[6];
+    q[0] = R.x[1];
+    q[1] = R.x[2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q[2 + i] = R.v[i];
+    bool acc;
+    double h_used = 0.0;
+    StepEnd end;
+    attempt_dp45_fp64<kMetricKerr>(P, R, K, k1v, k7p, acc, h_used, end);
+    ++tries;
+    if (acc) {
+      double* const o = rec + (uint64_t)j * (kRecDoubles * 32);
+#pragma unroll
+      for (int c = 0; c < 6; ++c) o[c * 32] = q[c];
+      const bool refl = end.xraw[2] < 0.0 || end.xraw[2] > kPi;
+      o[6 * 32] = refl ? -h_used : h_used;
+#pragma unroll
+      for (int l = 0; l < 6; ++l) {
+        double k[4];
+        K.get(l, k);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[(7 + 4 * l + i) * 32] = k[i];
+      }
+      ++j;
+      tries = 0;
+    }
+  }
+}
+
+// The crossing steps of the window's rays: the adjoint at their start and the
+// direct parameter terms.
+__global__ void __launch_bounds__(64)
+    backward_crossing_kernel(const __grid_constant__ DevParams P, const __grid_constant__ DiffOut D,
+                             const double* dl_drgb, const __grid_constant__ BackwardWork W) {
+  const uint64_t n = W.e1 - W.e0, le = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (le >= n) return;
+  const BackwardEntry E = entry_at(W, W.e0 + le);
+  const uint64_t idx = W.list[E.e];
+  const double dl[3] = {dl_drgb[3 * idx], dl_drgb[3 * idx + 1], dl_drgb[3 * idx + 2]};
+  const uint32_t steps = segment_steps(D.rays[idx].n_acc, E.segs, E.segs - 1);
+  double lam[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  double ga = 0.0, g_rin = 0.0, g_q = 0.0, g_sobs = 0.0;
+  bool ok = steps > 0;
+  if (ok) {
+    const double* q = W.rec + rec_at(E.item + E.segs - 1 - W.g0, steps - 1, 0);
+    const double x[4] = {0.0, q[0], q[32], 0.0};
+    const double v[4] = {q[64], q[96], q[128], q[160]};
+    ok = crossing_vjp(P, x, v, fabs(q[192]), dl, lam, &ga, &g_rin, &g_q, &g_sobs);
+  }
+  const double out[kRayDoubles] = {lam[0], lam[1], lam[2], lam[3], lam[4], lam[5],
+                                   ga,     g_rin,  g_q,    g_sobs, ok ? 1.0 : 0.0};
+#pragma unroll
+  for (int c = 0; c < kRayDoubles; ++c) W.ray[c * n + le] = out[c];
+}
+
+// Back through `steps` recorded steps of one item, the last first.
+GG_DEV void chain_segment(const DevParams& P, const BackwardWork& W, const ChainStore& C,
+                          uint64_t item, uint32_t steps, double lx[2], double lv[4], double* ga) {
+  for (uint32_t j = steps; j-- > 0;) {
+    const double* q = W.rec + rec_at(item - W.g0, j, 0);
+    const double r = q[0], th = q[32], h = q[192];
+    const double v[4] = {q[64], q[96], q[128], q[160]};
+#pragma unroll
+    for (int l = 0; l < 6; ++l) {
+      double k[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) k[i] = q[(7 + 4 * l + i) * 32];
+      C.set_k(l, k);
+    }
+    if (h < 0.0) lx[1] = -lx[1];  // theta -> -theta or 2 pi - theta
+    step_vjp(P, C, r, th, v, fabs(h), lx, lv, ga);
+  }
+}
+
+// Blocks below `tail_blocks` take the window's rays, a lane each, through
+// their last segments; the others the parallel segments, six lanes each.
+__global__ void __launch_bounds__(kChainBlock, kChainMinBlocks)
+    backward_chain_kernel(const __grid_constant__ DevParams P, const __grid_constant__ DiffOut D,
+                          const __grid_constant__ BackwardWork W, unsigned tail_blocks) {
+  __shared__ double2 k_smem[6][2][kChainBlock];
+  __shared__ double2 x_smem[6][3][kChainBlock];
+  const ChainStore C{k_smem, x_smem};
+  if (blockIdx.x < tail_blocks) {
+    const uint64_t n = W.e1 - W.e0, le = (uint64_t)blockIdx.x * kChainBlock + threadIdx.x;
+    if (le >= n || W.ray[10 * n + le] == 0.0) return;
+    const BackwardEntry E = entry_at(W, W.e0 + le);
+    double lx[2], lv[4], ga = W.ray[6 * n + le];
+    lx[0] = W.ray[le];
+    lx[1] = W.ray[n + le];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) lv[i] = W.ray[(2 + i) * n + le];
+    const uint32_t par = parallel_segments(W, E.segs);
+    for (uint32_t seg = E.segs; seg-- > par;) {
+      const bool last = seg + 1 == E.segs;  // its last step is the crossing
+      const uint32_t steps =
+          last ? segment_steps(D.rays[W.list[E.e]].n_acc, E.segs, seg) - 1 : (uint32_t)kCkptEvery;
+      chain_segment(P, W, C, E.item + seg, steps, lx, lv, &ga);
+    }
+    W.ray[le] = lx[0];
+    W.ray[n + le] = lx[1];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) W.ray[(2 + i) * n + le] = lv[i];
+    W.ray[6 * n + le] = ga;
+  } else {
+    const uint64_t t = (uint64_t)(blockIdx.x - tail_blocks) * kChainBlock + threadIdx.x;
+    const uint64_t p = W.p0 + t / 6;
+    const int c = (int)(t % 6);
+    if (p >= W.p1) return;
+    const BackwardBin& b = W.bins[find_bin<&BackwardBin::par>(W, p)];
+    const uint32_t per = parallel_segments(W, b.segs);  // > 0 in the bin that holds p
+    const uint64_t in_bin = p - b.par;
+    const uint64_t item = b.item + in_bin / per * b.segs + in_bin % per;
+    double lx[2] = {c == 0 ? 1.0 : 0.0, c == 1 ? 1.0 : 0.0};
+    double lv[4] = {c == 2 ? 1.0 : 0.0, c == 3 ? 1.0 : 0.0, c == 4 ? 1.0 : 0.0,
+                    c == 5 ? 1.0 : 0.0};
+    double ga = 0.0;
+    chain_segment(P, W, C, item, (uint32_t)kCkptEvery, lx, lv, &ga);
+    double* o = W.par + ((p - W.p0) * 6 + c) * 7;
+    o[0] = lx[0];
+    o[1] = lx[1];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[2 + i] = lv[i];
+    o[6] = ga;
+  }
+}
+
+// The adjoints of the window's rays at their camera states, through the
+// parallel segments' Jacobians, then the camera; the five sums into grad5.
+__global__ void __launch_bounds__(128)
+    backward_camera_kernel(const __grid_constant__ DevParams P, const __grid_constant__ BackwardWork W,
+                           double* grad5) {
   double acc5[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  const unsigned lane = threadIdx.x & 31u;
-  const uint64_t n = *L.total;
-  for (;;) {
-    unsigned long long b = 0;
-    if (lane == 0) b = atomicAdd(L.head, 32ull);
-    b = __shfl_sync(kFull, b, 0);
-    if (b >= n) break;
-    if (b + lane < n) backward_ray(P, D, dl_drgb, L.list[b + lane], acc5);
+  const uint64_t n = W.e1 - W.e0;
+  for (uint64_t le = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; le < n;
+       le += (uint64_t)gridDim.x * blockDim.x) {
+    if (W.ray[10 * n + le] == 0.0) continue;
+    const BackwardEntry E = entry_at(W, W.e0 + le);
+    double l[6], ga = W.ray[6 * n + le];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) l[c] = W.ray[c * n + le];
+    for (uint32_t seg = parallel_segments(W, E.segs); seg-- > 0;) {
+      const double* m = W.par + (E.par + seg - W.p0) * 42;
+      double t[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int c = 0; c < 6; ++c)
+#pragma unroll
+        for (int d = 0; d < 7; ++d) t[d] = fma(l[c], m[7 * c + d], t[d]);
+#pragma unroll
+      for (int c = 0; c < 6; ++c) l[c] = t[c];
+      ga += t[6];
+    }
+    double u, v;
+    sample_uv(P, W.list[E.e], u, v);
+    Dual<3> y0[8], sobs;
+    camera_dual(P, u, v, y0, &sobs);
+    constexpr int kComp[6] = {1, 2, 4, 5, 6, 7};
+    const double g_sobs = W.ray[9 * n + le];
+    double g3[3] = {ga, 0.0, 0.0};
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+#pragma unroll
+      for (int c = 0; c < 6; ++c) g3[p] += l[c] * y0[kComp[c]].d[p];
+      g3[p] += g_sobs * sobs.d[p];
+    }
+    acc5[0] += g3[0];
+    acc5[1] += g3[1];
+    acc5[2] += g3[2];
+    acc5[3] += W.ray[7 * n + le];
+    acc5[4] += W.ray[8 * n + le];
   }
 #pragma unroll
   for (int p = 0; p < 5; ++p) {
@@ -557,34 +693,128 @@ __global__ void __launch_bounds__(128, GG_ADJ_MIN_BLOCKS) diff_backward_kernel(c
   }
 }
 
-}  // namespace
+unsigned blocks_for(uint64_t n, unsigned per) { return (unsigned)((n + per - 1) / per); }
 
-size_t backward_list_bytes(uint64_t n_rays, uint32_t n_keys) {
-  return 16 + ((4 * (size_t)n_keys + 7) & ~size_t(7)) + 8 * n_rays;
+unsigned list_grid(const DevParams& P, int sms) {
+  const uint64_t need = (P.n_rays + 255) / 256, cap = (uint64_t)sms * 8;
+  return (unsigned)(need < cap ? (need < 1 ? 1 : need) : cap);
 }
 
-cudaError_t launch_diff_backward(const DevParams& P, const DiffOut& D, const double* dl_drgb,
-                                 double* grad5, void* list_buf, int sms, cudaStream_t stream) {
-  char* base = static_cast<char*>(list_buf);
-  BackwardList L;
-  L.head = reinterpret_cast<unsigned long long*>(base);
-  L.total = reinterpret_cast<uint32_t*>(base + 8);
-  L.bins = reinterpret_cast<uint32_t*>(base + 16);
-  L.list = reinterpret_cast<uint64_t*>(base + 16 + ((4 * (size_t)D.ckpt_per_ray + 7) & ~size_t(7)));
-  L.n_keys = D.ckpt_per_ray;
-  cudaError_t e = cudaMemsetAsync(base, 0, 16 + 4 * (size_t)D.ckpt_per_ray, stream);
+}  // namespace
+
+cudaError_t launch_backward_count(const DevParams& P, const DiffOut& D, const double* dl_drgb,
+                                  uint32_t* bins, int sms, cudaStream_t stream) {
+  const cudaError_t e =
+      cudaMemsetAsync(bins, 0, sizeof(uint32_t) * (size_t)D.ckpt_per_ray, stream);
   if (e != cudaSuccess) return e;
-  const uint64_t blocks_needed = (P.n_rays + 255) / 256;
-  uint64_t grid = (uint64_t)sms * 8;
-  if (grid > blocks_needed) grid = blocks_needed;
-  if (grid < 1) grid = 1;
-  backward_count_kernel<<<(unsigned)grid, 256, 0, stream>>>(P, D, dl_drgb, L);
-  backward_scan_kernel<<<1, kScanThreads, 0, stream>>>(L);
-  backward_scatter_kernel<<<(unsigned)grid, 256, 0, stream>>>(P, D, dl_drgb, L);
-  int bps = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, diff_backward_kernel, 128, 0);
-  if (e != cudaSuccess) return e;
-  diff_backward_kernel<<<sms * (bps > 0 ? bps : 1), 128, 0, stream>>>(P, D, dl_drgb, grad5, L);
+  backward_count_kernel<<<list_grid(P, sms), 256, 0, stream>>>(P, D, dl_drgb, bins);
+  return cudaGetLastError();
+}
+
+size_t backward_bins_bytes(uint32_t n_keys) { return sizeof(BackwardBin) * ((size_t)n_keys + 1); }
+
+BackwardPlan backward_plan(const uint32_t* counts, uint32_t n_keys, uint64_t* next, void* bins) {
+  auto* b = static_cast<BackwardBin*>(bins);
+  BackwardPlan plan{};
+  uint64_t listed = 0;
+  for (uint32_t k = 0; k < n_keys; ++k) listed += counts[k];
+  // An earlier segment costs six lanes' work where the ray's own lane would take
+  // it in sequence: with fewer rays than lanes (37,888) the chain is what
+  // counts, with more the work.  Backward ms at 1 / 2 / 3 / 4 / 5 segments in
+  // sequence, by listed rays: 1,800 (64^2) 0.50 / 0.66 / 0.83 / 1.00 / 1.16, 7,000
+  // (128^2) 0.76 / 0.72 / 0.89 / 1.05 / 1.22, 17,000 1.28 / 0.96 / 1.03 / 1.20 / 1.33,
+  // 28,000 1.86 / 1.21 / 1.17 / 1.35 / 1.52, 44,000 2.77 / 1.75 / 1.59 / 1.63 / 1.79,
+  // 112,000 (512^2) 6.40 / 3.72 / 3.16 / 3.01 / 2.96.
+  plan.tail = listed <= 4096 ? 1 : listed <= 24576 ? 2 : listed <= 65536 ? 3 : 4;
+  for (uint32_t k = 0; k < n_keys; ++k) {
+    next[k] = plan.entries;
+    if (!counts[k]) continue;
+    const uint32_t segs = n_keys - k;
+    b[plan.bins++] = BackwardBin{plan.entries, plan.items, plan.par, segs, 0u};
+    const uint64_t par = segs > plan.tail ? segs - plan.tail : 0u;
+    plan.entries += counts[k];
+    plan.items += (uint64_t)counts[k] * segs;
+    plan.par += (uint64_t)counts[k] * par;
+  }
+  b[plan.bins] = BackwardBin{plan.entries, plan.items, plan.par, 1u, 0u};
+  return plan;
+}
+
+// The window that starts at entry e0 and holds at most `most` items (one entry
+// at least).
+BackwardWindow backward_window(const void* bins, const BackwardPlan& plan, uint64_t e0,
+                               uint64_t most) {
+  const auto* b = static_cast<const BackwardBin*>(bins);
+  BackwardWindow w{};
+  bool begun = false;
+  for (uint32_t k = 0; k < plan.bins; ++k) {
+    const uint64_t stop = b[k + 1].start;
+    if (e0 >= stop) continue;
+    const uint64_t from = e0 > b[k].start ? e0 - b[k].start : 0;
+    const uint64_t par = b[k].segs > plan.tail ? b[k].segs - plan.tail : 0u;
+    if (!begun) {
+      w.e0 = e0;
+      w.g0 = b[k].item + from * b[k].segs;
+      w.p0 = b[k].par + from * par;
+      w.e1 = w.e0;
+      w.g1 = w.g0;
+      w.p1 = w.p0;
+      begun = true;
+    }
+    const uint64_t have = stop - b[k].start - from, left = most - (w.g1 - w.g0);
+    uint64_t take = left / b[k].segs;
+    if (take > have) take = have;
+    if (take == 0 && w.e1 == w.e0) take = 1;
+    w.e1 += take;
+    w.g1 += take * b[k].segs;
+    w.p1 += take * par;
+    if (take < have) break;
+  }
+  return w;
+}
+
+size_t backward_rec_bytes(uint64_t items) {
+  return ((items + 31) / 32) * 32 * sizeof(double) * kCkptEvery * kRecDoubles;
+}
+size_t backward_ray_bytes(uint64_t entries, uint64_t par) {
+  return sizeof(double) * (kRayDoubles * entries + 42 * par);
+}
+
+cudaError_t launch_backward_scatter(const DevParams& P, const DiffOut& D, const double* dl_drgb,
+                                    uint64_t* next, uint64_t* list, int sms,
+                                    cudaStream_t stream) {
+  backward_scatter_kernel<<<list_grid(P, sms), 256, 0, stream>>>(
+      P, D, dl_drgb, reinterpret_cast<unsigned long long*>(next), list);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_backward_window(const DevParams& P, const DiffOut& D, const double* dl_drgb,
+                                   const uint64_t* list, const void* bins, const BackwardPlan& plan,
+                                   const BackwardWindow& w, double* rec, double* ray,
+                                   double* grad5, int sms, cudaStream_t stream) {
+  BackwardWork W{};
+  W.list = list;
+  W.bins = static_cast<const BackwardBin*>(bins);
+  W.n_bins = plan.bins;
+  W.tail = plan.tail;
+  W.e0 = w.e0;
+  W.e1 = w.e1;
+  W.g0 = w.g0;
+  W.g1 = w.g1;
+  W.p0 = w.p0;
+  W.p1 = w.p1;
+  W.rec = rec;
+  W.ray = ray;
+  W.par = ray + kRayDoubles * (w.e1 - w.e0);
+  const uint64_t n = w.e1 - w.e0;
+  if (n == 0) return cudaSuccess;
+  backward_replay_kernel<<<blocks_for(w.g1 - w.g0, kTraceBlock), kTraceBlock, 0, stream>>>(P, D, W);
+  backward_crossing_kernel<<<blocks_for(n, 64), 64, 0, stream>>>(P, D, dl_drgb, W);
+  const unsigned tail = blocks_for(n, kChainBlock);
+  backward_chain_kernel<<<tail + blocks_for((w.p1 - w.p0) * 6, kChainBlock), kChainBlock, 0,
+                          stream>>>(P, D, W, tail);
+  const unsigned cam = blocks_for(n, 128), cap = (unsigned)sms * 8;
+  backward_camera_kernel<<<cam < cap ? cam : cap, 128, 0, stream>>>(P, W, grad5);
   return cudaGetLastError();
 }
 

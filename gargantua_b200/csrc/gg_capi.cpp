@@ -68,8 +68,18 @@ struct gg_ctx {
   size_t diff_rays_cap = 0;
   void* diff_ckpt = nullptr;
   size_t diff_ckpt_cap = 0;
-  void* diff_list = nullptr;  // the backward pass's sorted work list
+  // the backward pass: keys' counters and bins (device and pinned mirror), the
+  // sorted work list, step records, per-ray and per-segment results
+  void* diff_keys = nullptr;
+  size_t diff_keys_cap = 0;
+  void* diff_keys_host = nullptr;
+  size_t diff_keys_host_cap = 0;
+  void* diff_list = nullptr;
   size_t diff_list_cap = 0;
+  void* diff_rec = nullptr;
+  size_t diff_rec_cap = 0;
+  void* diff_ray = nullptr;
+  size_t diff_ray_cap = 0;
   double* diff_grad = nullptr;       // 5 doubles, device
   double* diff_grad_host = nullptr;  // pinned
   // equirectangular sky map (gg_set_hdri), RGB float texels on the device
@@ -939,7 +949,11 @@ GG_API int gg_destroy(gg_ctx* c) {
   if (c->batch_host) cudaFreeHost(c->batch_host);
   if (c->diff_rays) cudaFree(c->diff_rays);
   if (c->diff_ckpt) cudaFree(c->diff_ckpt);
+  if (c->diff_keys) cudaFree(c->diff_keys);
+  if (c->diff_keys_host) cudaFreeHost(c->diff_keys_host);
   if (c->diff_list) cudaFree(c->diff_list);
+  if (c->diff_rec) cudaFree(c->diff_rec);
+  if (c->diff_ray) cudaFree(c->diff_ray);
   if (c->diff_grad) cudaFree(c->diff_grad);
   if (c->diff_grad_host) cudaFreeHost(c->diff_grad_host);
   if (c->hdri) cudaFree(c->hdri);
@@ -1216,17 +1230,63 @@ GG_API int gg_backward(gg_ctx* c, const double* dl_drgb_dev, double grad[5], voi
     c->diff_grad_host = nullptr;
     return GG_ERR_OOM;
   }
-  const int gl = grow(&c->diff_list, &c->diff_list_cap,
-                     gg::backward_list_bytes(c->diff_P.n_rays, c->diff_ckpt_per_ray));
-  if (gl != GG_OK) return gl;
+  const uint32_t n_keys = c->diff_ckpt_per_ray;
+  // layout of the keys' block: first places, bins, counters
+  const size_t next_bytes = align256(sizeof(uint64_t) * n_keys);
+  const size_t bins_bytes = align256(gg::backward_bins_bytes(n_keys));
+  const size_t keys_bytes = next_bytes + bins_bytes + sizeof(uint32_t) * n_keys;
+  int st = grow(&c->diff_keys, &c->diff_keys_cap, keys_bytes);
+  if (st != GG_OK) return st;
+  st = grow_pinned(&c->diff_keys_host, &c->diff_keys_host_cap, keys_bytes);
+  if (st != GG_OK) return st;
+  char* kd = static_cast<char*>(c->diff_keys);
+  char* kh = static_cast<char*>(c->diff_keys_host);
   gg::DiffOut D{static_cast<gg::DiffRay*>(c->diff_rays), static_cast<gg::Ckpt*>(c->diff_ckpt),
-                c->diff_ckpt_per_ray, 0u};
+                n_keys, 0u};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (cudaStreamWaitEvent(s, c->ev_done, 0) != cudaSuccess) return GG_ERR_CUDA;
   if (cudaMemsetAsync(c->diff_grad, 0, 5 * sizeof(double), s) != cudaSuccess) return GG_ERR_CUDA;
-  if (gg::launch_diff_backward(c->diff_P, D, dl_drgb_dev, c->diff_grad, c->diff_list, c->sms,
-                               s) != cudaSuccess)
+  auto* counts = reinterpret_cast<uint32_t*>(kh + next_bytes + bins_bytes);
+  if (gg::launch_backward_count(c->diff_P, D, dl_drgb_dev,
+                                reinterpret_cast<uint32_t*>(kd + next_bytes + bins_bytes), c->sms,
+                                s) != cudaSuccess ||
+      cudaMemcpyAsync(counts, kd + next_bytes + bins_bytes, sizeof(uint32_t) * n_keys,
+                      cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+      cudaStreamSynchronize(s) != cudaSuccess)
     return GG_ERR_CUDA;
+  const gg::BackwardPlan plan = gg::backward_plan(
+      counts, n_keys, reinterpret_cast<uint64_t*>(kh), kh + next_bytes);
+  if (plan.entries) {
+    st = grow(&c->diff_list, &c->diff_list_cap, sizeof(uint64_t) * plan.entries);
+    if (st != GG_OK) return st;
+    gg::BackwardWindow w{};
+    uint64_t items = 0;
+    size_t ray_bytes = 0;
+    for (uint64_t e = 0; e < plan.entries; e = w.e1) {
+      w = gg::backward_window(kh + next_bytes, plan, e, gg::kBackwardItems);
+      if (w.g1 - w.g0 > items) items = w.g1 - w.g0;
+      const size_t rb = gg::backward_ray_bytes(w.e1 - w.e0, w.p1 - w.p0);
+      if (rb > ray_bytes) ray_bytes = rb;
+    }
+    st = grow(&c->diff_rec, &c->diff_rec_cap, gg::backward_rec_bytes(items));
+    if (st != GG_OK) return st;
+    st = grow(&c->diff_ray, &c->diff_ray_cap, ray_bytes);
+    if (st != GG_OK) return st;
+    if (cudaMemcpyAsync(kd, kh, next_bytes + bins_bytes, cudaMemcpyHostToDevice, s) !=
+            cudaSuccess ||
+        gg::launch_backward_scatter(c->diff_P, D, dl_drgb_dev, reinterpret_cast<uint64_t*>(kd),
+                                    static_cast<uint64_t*>(c->diff_list), c->sms,
+                                    s) != cudaSuccess)
+      return GG_ERR_CUDA;
+    for (uint64_t e = 0; e < plan.entries; e = w.e1) {
+      w = gg::backward_window(kh + next_bytes, plan, e, gg::kBackwardItems);
+      if (gg::launch_backward_window(
+              c->diff_P, D, dl_drgb_dev, static_cast<const uint64_t*>(c->diff_list),
+              kd + next_bytes, plan, w, static_cast<double*>(c->diff_rec),
+              static_cast<double*>(c->diff_ray), c->diff_grad, c->sms, s) != cudaSuccess)
+        return GG_ERR_CUDA;
+    }
+  }
   if (cudaMemcpyAsync(c->diff_grad_host, c->diff_grad, 5 * sizeof(double),
                       cudaMemcpyDeviceToHost, s) != cudaSuccess)
     return GG_ERR_CUDA;

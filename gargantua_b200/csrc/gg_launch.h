@@ -104,13 +104,38 @@ cudaError_t launch_queue_trace(const DevParams& P, const DevOutputs& O, DevContr
                                int grid, cudaStream_t stream,
                                const BatchTable* batch = nullptr);
 
-// Differentiable render: the adjoint pass (gg_adjoint.cu) of a forward run
-// by launch_trace with P.ckpt set; grad5 (device) accumulates dL/d(a,
-// inclination, r_cam, r_inner, q).
-// list_buf (device, backward_list_bytes) holds the pass's sorted work list.
-size_t backward_list_bytes(uint64_t n_rays, uint32_t n_keys);
-cudaError_t launch_diff_backward(const DevParams& P, const DiffOut& D, const double* dl_drgb,
-                                 double* grad5, void* list_buf, int sms, cudaStream_t stream);
+// Differentiable render: the adjoint pass (gg_adjoint.cu) of a forward run by
+// launch_trace with P.ckpt set.  The disk rays with a nonzero dL/d(colour) are
+// counted per key (the checkpoint counts; bins: one counter per key), the host
+// lays the sorted list out (backward_plan: each key's first place into `next`,
+// the non-empty bins into `bins`), launch_backward_scatter fills it, and each
+// window of at most kBackwardItems segments is taken back, its sums added to
+// grad5 (device): dL/d(a, inclination, r_cam, r_inner, q).
+struct BackwardPlan {
+  uint64_t entries, items, par;  // rays, their segments, and those taken in parallel
+  uint32_t bins;                 // non-empty keys
+  uint32_t tail;                 // segments of a ray taken in sequence by one lane
+};
+struct BackwardWindow {
+  uint64_t e0, e1, g0, g1, p0, p1;
+};
+// Segments of a window: 2.1 GB of step records, one window for most images of
+// 512^2.
+constexpr uint64_t kBackwardItems = 1ull << 18;
+cudaError_t launch_backward_count(const DevParams& P, const DiffOut& D, const double* dl_drgb,
+                                  uint32_t* bins, int sms, cudaStream_t stream);
+size_t backward_bins_bytes(uint32_t n_keys);
+BackwardPlan backward_plan(const uint32_t* counts, uint32_t n_keys, uint64_t* next, void* bins);
+BackwardWindow backward_window(const void* bins, const BackwardPlan& plan, uint64_t e0,
+                               uint64_t most);
+size_t backward_rec_bytes(uint64_t items);
+size_t backward_ray_bytes(uint64_t entries, uint64_t par);
+cudaError_t launch_backward_scatter(const DevParams& P, const DiffOut& D, const double* dl_drgb,
+                                    uint64_t* next, uint64_t* list, int sms, cudaStream_t stream);
+cudaError_t launch_backward_window(const DevParams& P, const DiffOut& D, const double* dl_drgb,
+                                   const uint64_t* list, const void* bins, const BackwardPlan& plan,
+                                   const BackwardWindow& w, double* rec, double* ray,
+                                   double* grad5, int sms, cudaStream_t stream);
 
 // Best-of-5 FMA throughput (FLOP/s, FMA = 2) of the current device.
 cudaError_t measure_fma_peak(int fp64, int sms, double* flops);
