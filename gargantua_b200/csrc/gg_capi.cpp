@@ -508,25 +508,21 @@ int enqueue(gg_ctx* ctx, const DevParams& P, DevOutputs O, bool want_image,
     if (st != GG_OK) return st;
     O.chain = static_cast<gg::ChainRay*>(ctx->chain);
   }
-  int qbps = 0, rbps = 0;
-  if (mixed && (gg::queue_trace_occupancy(P, &qbps) != cudaSuccess || qbps < 1))
-    return GG_ERR_CUDA;
+  int rbps = 0;
   if (rounds && (gg::mixed_occupancy(P, &rbps, nullptr, 0, true) != cudaSuccess || rbps < 1))
     return GG_ERR_CUDA;
   if (cudaEventRecord(ctx->ev_start, stream) != cudaSuccess) return GG_ERR_CUDA;
   if (mixed) {
     if (gg::launch_mixed(P, O, ctx->ctl, (int)grid, stream) != cudaSuccess) return GG_ERR_CUDA;
-    // the queues' lengths are only known on the device: full persistent
-    // grids, whose surplus warps find the queue empty and exit
     DevParams P1 = P;
     P1.hand_back = rounds ? 1u : 0u;
-    if (gg::launch_queue_trace(P1, O, ctx->ctl, ctx->sms * qbps, stream) != cudaSuccess)
+    if (gg::launch_queue_trace(P1, O, ctx->ctl, ctx->sms, stream) != cudaSuccess)
       return GG_ERR_CUDA;
     if (rounds) {
       if (gg::launch_next_round(ctx->ctl, stream) != cudaSuccess ||
           gg::launch_mixed(P, O, ctx->ctl, ctx->sms * rbps, stream, nullptr, 0, true) !=
               cudaSuccess ||
-          gg::launch_queue_trace(P, O, ctx->ctl, ctx->sms * qbps, stream) != cudaSuccess)
+          gg::launch_queue_trace(P, O, ctx->ctl, ctx->sms, stream) != cudaSuccess)
         return GG_ERR_CUDA;
     }
   } else if (gg::launch_trace(P, O, ctx->ctl, (int)grid, stream) != cudaSuccess ||
@@ -581,7 +577,7 @@ struct BatchLaunch {
   size_t table_bytes = 0;  // bytes of the scene table + prefix array to upload
   uint64_t total = 0;
   uint64_t pixels = 0;
-  int grid = 0, qgrid = 0, rgrid = 0;
+  int grid = 0, rgrid = 0;
   bool rounds = false;  // hand rays back from the FP64 pass (kHandBackMinRays)
 };
 
@@ -649,10 +645,9 @@ int batch_prepare(gg_ctx* c, const gg_scene_t* scenes, uint32_t n, const gg_inte
   L->table.scenes = static_cast<const gg::BatchScene*>(c->batch_dev);
   L->table.first = reinterpret_cast<const uint64_t*>(static_cast<char*>(c->batch_dev) + off_first);
   L->table.n = n;
-  int bps = 0, qbps = 0;
+  int bps = 0;
   if (gg::mixed_occupancy(L->P0, &bps, &L->table, variant) != cudaSuccess || bps < 1)
     return GG_ERR_CUDA;
-  if (gg::queue_trace_occupancy(L->P0, &qbps) != cudaSuccess || qbps < 1) return GG_ERR_CUDA;
   int rbps = 0;
   if (gg::mixed_occupancy(L->P0, &rbps, &L->table, 0, true) != cudaSuccess || rbps < 1)
     return GG_ERR_CUDA;
@@ -661,7 +656,6 @@ int batch_prepare(gg_ctx* c, const gg_scene_t* scenes, uint32_t n, const gg_inte
   const uint64_t need_blocks = (total + gg::kTraceBlock - 1) / gg::kTraceBlock;
   if (grid > need_blocks) grid = need_blocks;
   L->grid = (int)(grid < 1 ? 1 : grid);
-  L->qgrid = c->sms * qbps;
   return GG_OK;
 }
 
@@ -679,12 +673,12 @@ int batch_body(gg_ctx* c, const BatchLaunch& L, int variant, cudaStream_t s) {
     return GG_ERR_CUDA;
   DevParams P1 = L.P0;
   P1.hand_back = L.rounds ? 1u : 0u;
-  if (gg::launch_queue_trace(P1, L.O0, c->ctl, L.qgrid, s, &L.table) != cudaSuccess)
+  if (gg::launch_queue_trace(P1, L.O0, c->ctl, c->sms, s, &L.table) != cudaSuccess)
     return GG_ERR_CUDA;
   if (L.rounds &&
       (gg::launch_next_round(c->ctl, s) != cudaSuccess ||
        gg::launch_mixed(L.P0, L.O0, c->ctl, L.rgrid, s, &L.table, 0, true) != cudaSuccess ||
-       gg::launch_queue_trace(L.P0, L.O0, c->ctl, L.qgrid, s, &L.table) != cudaSuccess))
+       gg::launch_queue_trace(L.P0, L.O0, c->ctl, c->sms, s, &L.table) != cudaSuccess))
     return GG_ERR_CUDA;
   if (cudaMemcpyAsync(c->ctl_host, c->ctl, sizeof(DevControl), cudaMemcpyDeviceToHost, s) !=
       cudaSuccess)

@@ -41,7 +41,10 @@ constexpr int kTraceMinBlocksKerrChain = 4;
 #endif
 constexpr int kTraceMinBlocksSchw = 4;
 #endif
-constexpr int kTraceMinBlocksGroup = 3;  // 168 registers: no spills, latency is all that counts
+// The group kernel and the unrolled full Dormand-Prince ones: 168 registers, few
+// or no spills.  At 4 / 3 / 2 CTAs the 128^2 forward takes 2.48 / 2.36 / 2.29 ms, the 321x181 mixed
+// preview 2.99 / 2.83 / 3.03.
+constexpr int kTraceMinBlocksGroup = 3;
 
 // Resident CTAs per SM the mixed-precision trace kernel is budgeted for: its
 // camera pass (8, 64 registers: throughput), and its pass over the rays the
@@ -99,10 +102,8 @@ cudaError_t launch_mixed(const DevParams& P, const DevOutputs& O, DevControl* ct
                          cudaStream_t stream, const BatchTable* batch = nullptr,
                          int variant = 0, bool returned = false);
 cudaError_t launch_next_round(DevControl* ctl, cudaStream_t stream);
-cudaError_t queue_trace_occupancy(const DevParams& P, int* blocks_per_sm);
-cudaError_t launch_queue_trace(const DevParams& P, const DevOutputs& O, DevControl* ctl,
-                               int grid, cudaStream_t stream,
-                               const BatchTable* batch = nullptr);
+cudaError_t launch_queue_trace(const DevParams& P, const DevOutputs& O, DevControl* ctl, int sms,
+                               cudaStream_t stream, const BatchTable* batch = nullptr);
 
 // Differentiable render: the adjoint pass (gg_adjoint.cu) of a forward run by
 // launch_trace with P.ckpt set.  The disk rays with a nonzero dL/d(colour) are

@@ -73,6 +73,17 @@ __device__ __noinline__ bool hand_to_group(const DevOutputs& O, DevControl* ctl,
   return true;
 }
 
+// How many rays a launch is for, which sets its register budget: many (a full
+// wave of lanes several times over), few per lane, or (full Dormand-Prince only)
+// so few that one ray's chain is the time -- then its stages are unrolled.
+enum : int { kSizeLarge = 0, kSizeSmall = 1, kSizeChain = 2 };
+
+// Band passes of at most this many rays take the unrolled form: about a ray a
+// lane.  Rolled / unrolled, mixed form, ms (band rays): 321x181 3.43 / 2.94 (1,700),
+// 500x320 4.70 / 4.18, 1100x800 12.7 / 12.2 (25,000), 1080p 24.0 / 23.7 (59,000), the near
+// view at 500^2 6.07 / 5.48 (27,000), 900^2 8.36 / 8.54 (86,000), 2048^2 x 4 83.1 / 86.9.
+constexpr unsigned long long kBandChainRays = 1ull << 16;
+
 // SRC: kSrcCamera traces the render's samples from the camera; kSrcQueue
 // finishes, in FP64, the rays the mixed-precision pass handed over (their
 // count is read from ctl->queued, which that pass wrote before this launch);
@@ -89,14 +100,16 @@ __device__ __noinline__ bool hand_to_group(const DevOutputs& O, DevControl* ctl,
 // (O.chain), else from the camera.  Without GROUP, a warp that finds no more
 // samples and has at most kHandLanes rays left hands those to that queue.
 template <int METRIC, int DISK, int STEPPER, int SRC, bool BATCH, bool SCENE, bool CKPT,
-          bool SMALL, bool GROUP>
+          int SIZE, bool GROUP>
 __global__ void __launch_bounds__(kTraceBlock,
-                                  GROUP                                 ? kTraceMinBlocksGroup
-                                  : METRIC != kMetricKerr               ? kTraceMinBlocksSchw
-                                  : (SRC == kSrcQueue || CKPT || SMALL) ? kTraceMinBlocksKerrChain
-                                                                        : kTraceMinBlocksKerr)
+                                  GROUP || SIZE == kSizeChain ? kTraceMinBlocksGroup
+                                  : METRIC != kMetricKerr     ? kTraceMinBlocksSchw
+                                  : (SRC == kSrcQueue || CKPT || SIZE == kSizeSmall)
+                                      ? kTraceMinBlocksKerrChain
+                                      : kTraceMinBlocksKerr)
     trace_fp64_kernel(const __grid_constant__ DevParams P, const __grid_constant__ DevOutputs O,
                       DevControl* ctl, const __grid_constant__ BatchTable B) {
+  if (SRC == kSrcQueue && (ctl->queued <= kBandChainRays) != (SIZE == kSizeChain)) return;
   const unsigned lane = threadIdx.x & 31u;
   const bool from_chain = GROUP && O.chain != nullptr;
   const uint64_t n_src =
@@ -291,7 +304,8 @@ __global__ void __launch_bounds__(kTraceBlock,
       StepEnd end;
       int res;
       if (STEPPER == kStepperDP45)
-        res = attempt_dp45_fp64<METRIC>(PL, R, K, k1_valid, k7_pending, acc, h_used, end);
+        res = attempt_dp45_fp64<METRIC, SIZE == kSizeChain>(
+            PL, R, K, k1_valid, k7_pending, acc, h_used, end);
       else if (GROUP)
         res = attempt_fp64_group<METRIC>(PL, R, role, k1, k1_valid, acc, h_used);
       else
@@ -559,15 +573,16 @@ __global__ void reduce_samples_kernel(const __grid_constant__ DevParams P, const
 }
 
 template <int METRIC, int DISK, int STEPPER, int SRC, bool BATCH = false, bool SCENE = false,
-          bool CKPT = false, bool SMALL = false, bool GROUP = false>
+          bool CKPT = false, int SIZE = kSizeLarge, bool GROUP = false>
 const void* trace_fn() {
   return reinterpret_cast<const void*>(
-      &trace_fp64_kernel<METRIC, DISK, STEPPER, SRC, BATCH, SCENE, CKPT, SMALL, GROUP>);
+      &trace_fp64_kernel<METRIC, DISK, STEPPER, SRC, BATCH, SCENE, CKPT, SIZE, GROUP>);
 }
 
 template <int METRIC, int DISK, bool SCENE = false>
 const void* group_fn() {
-  return trace_fn<METRIC, DISK, kStepperReference, kSrcCamera, false, SCENE, false, false, true>();
+  return trace_fn<METRIC, DISK, kStepperReference, kSrcCamera, false, SCENE, false, kSizeLarge,
+                  true>();
 }
 
 // The group kernel of a render with the reference's step.
@@ -605,69 +620,67 @@ constexpr uint64_t kSmallRender = 1ull << 20;
 
 // With a scene: no disk or the volumetric one (the reference's
 // render_with_scene and render_with_disk_and_scene).
-template <int STEPPER, bool SMALL>
-const void* select_scene_kerr(const DevParams& P) {
-  return P.disk == kDiskVolumetric
-             ? trace_fn<kMetricKerr, kDiskVolumetric, STEPPER, kSrcCamera, false, true, false,
-                        SMALL>()
-             : trace_fn<kMetricKerr, kDiskNone, STEPPER, kSrcCamera, false, true, false, SMALL>();
-}
-
-template <int STEPPER>
-const void* select_scene(const DevParams& P) {
-  if (P.metric == kMetricKerr)
-    return P.n_rays < kSmallRender ? select_scene_kerr<STEPPER, true>(P)
-                                   : select_scene_kerr<STEPPER, false>(P);
-  return P.disk == kDiskVolumetric
-             ? trace_fn<kMetricSchwarzschild, kDiskVolumetric, STEPPER, kSrcCamera, false, true>()
-             : trace_fn<kMetricSchwarzschild, kDiskNone, STEPPER, kSrcCamera, false, true>();
-}
-
-template <int STEPPER, bool SMALL>
-const void* select_disk_kerr(const DevParams& P) {
+template <int METRIC, int STEPPER, int SIZE>
+const void* select_disk(const DevParams& P) {
+  if (P.scene)
+    return P.disk == kDiskVolumetric
+               ? trace_fn<METRIC, kDiskVolumetric, STEPPER, kSrcCamera, false, true, false, SIZE>()
+               : trace_fn<METRIC, kDiskNone, STEPPER, kSrcCamera, false, true, false, SIZE>();
   if (P.disk == kDiskThin)
-    return trace_fn<kMetricKerr, kDiskThin, STEPPER, kSrcCamera, false, false, false, SMALL>();
+    return trace_fn<METRIC, kDiskThin, STEPPER, kSrcCamera, false, false, false, SIZE>();
   if (P.disk == kDiskVolumetric)
-    return trace_fn<kMetricKerr, kDiskVolumetric, STEPPER, kSrcCamera, false, false, false,
-                    SMALL>();
-  return trace_fn<kMetricKerr, kDiskNone, STEPPER, kSrcCamera, false, false, false, SMALL>();
+    return trace_fn<METRIC, kDiskVolumetric, STEPPER, kSrcCamera, false, false, false, SIZE>();
+  return trace_fn<METRIC, kDiskNone, STEPPER, kSrcCamera, false, false, false, SIZE>();
 }
 
 template <int STEPPER>
-const void* select_metric_disk(const DevParams& P) {
-  if (P.scene) return select_scene<STEPPER>(P);
+const void* select_metric(const DevParams& P) {
   if (P.metric == kMetricKerr)
-    return P.n_rays < kSmallRender ? select_disk_kerr<STEPPER, true>(P)
-                                   : select_disk_kerr<STEPPER, false>(P);
-  if (P.disk == kDiskThin) return trace_fn<kMetricSchwarzschild, kDiskThin, STEPPER, kSrcCamera>();
-  if (P.disk == kDiskVolumetric)
-    return trace_fn<kMetricSchwarzschild, kDiskVolumetric, STEPPER, kSrcCamera>();
-  return trace_fn<kMetricSchwarzschild, kDiskNone, STEPPER, kSrcCamera>();
+    return P.n_rays < kSmallRender ? select_disk<kMetricKerr, STEPPER, kSizeSmall>(P)
+                                   : select_disk<kMetricKerr, STEPPER, kSizeLarge>(P);
+  return select_disk<kMetricSchwarzschild, STEPPER, kSizeLarge>(P);
 }
 
+// Full Dormand-Prince camera passes of at most this many samples take the
+// unrolled form.  Rolled / unrolled, ms, the differentiable forward: 64^2 1.83 /
+// 1.52, 128^2 2.84 / 2.32, 160^2 2.26 / 1.98, 200^2 2.53 / 2.34, 230^2 2.90 /
+// 2.65, 256^2 3.16 / 3.39, 512^2 7.2 / 8.5.
+constexpr uint64_t kChainRays = 3ull << 14;
 const void* select_trace(const DevParams& P) {
   if (group_render(P)) return select_group(P);
+  const bool chain = P.stepper == kStepperDP45 && P.n_rays <= kChainRays;
   // gg_forward_ckpt admits only Kerr, the thin disk and the full stepper
   if (P.ckpt)
-    return trace_fn<kMetricKerr, kDiskThin, kStepperDP45, kSrcCamera, false, false, true>();
-  return P.stepper == kStepperDP45 ? select_metric_disk<kStepperDP45>(P)
-                                   : select_metric_disk<kStepperReference>(P);
+    return chain ? trace_fn<kMetricKerr, kDiskThin, kStepperDP45, kSrcCamera, false, false, true,
+                            kSizeChain>()
+                 : trace_fn<kMetricKerr, kDiskThin, kStepperDP45, kSrcCamera, false, false, true>();
+  if (chain)
+    return P.metric == kMetricKerr ? select_disk<kMetricKerr, kStepperDP45, kSizeChain>(P)
+                                   : select_disk<kMetricSchwarzschild, kStepperDP45, kSizeChain>(P);
+  return P.stepper == kStepperDP45 ? select_metric<kStepperDP45>(P)
+                                   : select_metric<kStepperReference>(P);
 }
 
 // The FP64 pass of the mixed form: full Dormand-Prince, thin disk or none.
-template <bool BATCH>
-const void* select_queue_trace_b(const DevParams& P) {
-  if (P.metric == kMetricKerr)
-    return P.disk == kDiskThin
-               ? trace_fn<kMetricKerr, kDiskThin, kStepperDP45, kSrcQueue, BATCH>()
-               : trace_fn<kMetricKerr, kDiskNone, kStepperDP45, kSrcQueue, BATCH>();
+template <int METRIC, bool BATCH, int SIZE>
+const void* queue_fn(const DevParams& P) {
   return P.disk == kDiskThin
-             ? trace_fn<kMetricSchwarzschild, kDiskThin, kStepperDP45, kSrcQueue, BATCH>()
-             : trace_fn<kMetricSchwarzschild, kDiskNone, kStepperDP45, kSrcQueue, BATCH>();
+             ? trace_fn<METRIC, kDiskThin, kStepperDP45, kSrcQueue, BATCH, false, false, SIZE>()
+             : trace_fn<METRIC, kDiskNone, kStepperDP45, kSrcQueue, BATCH, false, false, SIZE>();
 }
 
-const void* select_queue_trace(const DevParams& P, bool batch) {
-  return batch ? select_queue_trace_b<true>(P) : select_queue_trace_b<false>(P);
+template <bool BATCH, int SIZE>
+const void* select_queue_metric(const DevParams& P) {
+  return P.metric == kMetricKerr ? queue_fn<kMetricKerr, BATCH, SIZE>(P)
+                                 : queue_fn<kMetricSchwarzschild, BATCH, SIZE>(P);
+}
+
+const void* select_queue_trace(const DevParams& P, bool batch, bool chain) {
+  if (chain)
+    return batch ? select_queue_metric<true, kSizeChain>(P)
+                 : select_queue_metric<false, kSizeChain>(P);
+  return batch ? select_queue_metric<true, kSizeLarge>(P)
+               : select_queue_metric<false, kSizeLarge>(P);
 }
 
 }  // namespace
@@ -675,11 +688,6 @@ const void* select_queue_trace(const DevParams& P, bool batch) {
 cudaError_t trace_occupancy(const DevParams& P, int* blocks_per_sm) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, select_trace(P),
                                                        kTraceBlock, 0);
-}
-
-cudaError_t queue_trace_occupancy(const DevParams& P, int* blocks_per_sm) {
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      blocks_per_sm, select_queue_trace(P, false), kTraceBlock, 0);
 }
 
 int chain_capacity(const DevParams& P, int grid) {
@@ -709,15 +717,26 @@ cudaError_t launch_group(const DevParams& P, const DevOutputs& O, DevControl* ct
   return cudaLaunchKernel(fn, dim3(grid), dim3(kTraceBlock), args, 0, stream);
 }
 
-cudaError_t launch_queue_trace(const DevParams& P, const DevOutputs& O, DevControl* ctl,
-                               int grid, cudaStream_t stream, const BatchTable* batch) {
-  const void* fn = select_queue_trace(P, batch != nullptr);
+cudaError_t launch_queue_trace(const DevParams& P, const DevOutputs& O, DevControl* ctl, int sms,
+                               cudaStream_t stream, const BatchTable* batch) {
   DevParams p = P;
   DevOutputs o = O;
   BatchTable b{};
   if (batch) b = *batch;
   void* args[] = {&p, &o, &ctl, &b};
-  return cudaLaunchKernel(fn, dim3(grid), dim3(kTraceBlock), args, 0, stream);
+  // The queue's length is only known on the device: both forms are launched,
+  // full persistent grids, and the one it is not for returns at once.
+  for (int chain = 1; chain >= 0; --chain) {
+    if (!chain && O.queue_cap <= kBandChainRays) break;
+    const void* fn = select_queue_trace(P, batch != nullptr, chain != 0);
+    int bps = 0;
+    const cudaError_t q = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, kTraceBlock, 0);
+    if (q != cudaSuccess) return q;
+    const cudaError_t e = cudaLaunchKernel(fn, dim3(sms * (bps > 0 ? bps : 1)),
+                                           dim3(kTraceBlock), args, 0, stream);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 cudaError_t launch_trace(const DevParams& P, const DevOutputs& O, DevControl* ctl, int grid,
