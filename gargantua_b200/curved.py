@@ -374,6 +374,25 @@ class RayOutputs:
         self.rgb = np.zeros((n, 3), np.float64)
         self.cross = np.zeros((8, n), np.float64)
 
+    @classmethod
+    def _to_fill(cls, n: int) -> "RayOutputs":
+        """The same arrays without initial values, for a render that writes
+        every entry: filling 13 MB (256^2 samples) first, in pages the system
+        has to clear, took 1.2 of the call's 4.2 ms."""
+        o = cls.__new__(cls)
+        o.n = n
+        o.cls = np.empty(n, np.int32)
+        o.x = np.empty((4, n), np.float64)
+        o.v = np.empty((4, n), np.float64)
+        o.lam = np.empty(n, np.float64)
+        o.attempts = np.empty(n, np.uint32)
+        o.accepted = np.empty(n, np.uint32)
+        o.intensity = np.empty(n, np.float64)
+        o.color_temp = np.empty(n, np.float64)
+        o.rgb = np.empty((n, 3), np.float64)
+        o.cross = np.empty((8, n), np.float64)
+        return o
+
     def struct(self) -> abi.gg_ray_out_t:
         def p(a, t):
             return a.ctypes.data_as(C.POINTER(t))
@@ -436,8 +455,9 @@ class Renderer:
 
     def render(self, scene: Scene, rays: bool = False):
         """Synchronous render into host memory: (image, RayOutputs or None)."""
-        img = np.zeros((scene.rows, scene.width, 3), np.uint8)
-        out = RayOutputs(scene.n_samples) if rays else None
+        # gg_render copies whole arrays back or fails
+        img = np.empty((scene.rows, scene.width, 3), np.uint8)
+        out = RayOutputs._to_fill(scene.n_samples) if rays else None
         self._sky_map(scene)
         st = self._lib.gg_render(self._h, *scene.c_args(), img.ctypes.data_as(C.c_void_p),
                                  C.byref(out.struct()) if out else None)
@@ -493,7 +513,7 @@ class Renderer:
     def render_batch(self, scenes) -> list:
         """Synchronous batched render (gg_render_batch): one image per scene."""
         arr, integ, opts, _ = self._batch_structs(scenes)
-        imgs = [np.zeros((sc.height, sc.width, 3), np.uint8) for sc in scenes]
+        imgs = [np.empty((sc.height, sc.width, 3), np.uint8) for sc in scenes]
         ptrs = (C.c_void_p * len(scenes))(*[im.ctypes.data for im in imgs])
         abi.check(self._lib.gg_render_batch(self._h, arr, len(scenes), C.byref(integ),
                                             C.byref(opts), ptrs), "gg_render_batch")
