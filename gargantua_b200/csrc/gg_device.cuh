@@ -596,8 +596,9 @@ GG_DEV bool end_attempt_fp64(const DevParams& P, Ray& R, const double nv[4], con
 
 // One call of RK45Integrator::step (geodesic.rs:185-328) in FP64.
 // Returns the StepResult; `accepted` and `h_used` describe an advance.
-template <int METRIC>
+template <int METRIC, bool UNROLL>
 //
+// UNROLL: see attempt_dp45_fp64.
 // `k1_valid` says K(0, .) already holds a(x, v) for the current state: the
 // reference's k7 is evaluated at (pos + h vel, new_vel), exactly the state an
 // accepted step moves to, so it is the next attempt's k1 (first same as
@@ -638,8 +639,7 @@ GG_DEV int attempt_fp64(const DevParams& P, Ray& R, const KStore& K, bool& k1_va
   // k1 is valid keeps its own (the previous step's k7), so that a ray's
   // result does not depend on which rays share its warp.
   const int s_first = __any_sync(__activemask(), !k1_valid) ? 0 : 1;
-#pragma unroll 1
-  for (int s = s_first; s < 6; ++s) {
+  auto stage = [&](int s) {
     double w[4], a[4];
     switch (s) {
       case 0:
@@ -670,6 +670,14 @@ GG_DEV int attempt_fp64(const DevParams& P, Ray& R, const KStore& K, bool& k1_va
     } else if (s > 0 || !k1_valid) {
       K.set(s, a);
     }
+  };
+  if (UNROLL) {
+    if (s_first == 0) stage(0);
+#pragma unroll
+    for (int s = 1; s < 6; ++s) stage(s);
+  } else {
+#pragma unroll 1
+    for (int s = s_first; s < 6; ++s) stage(s);
   }
   k1_valid = true;  // a rejected attempt leaves the state, so k1 stays
 

@@ -74,8 +74,8 @@ __device__ __noinline__ bool hand_to_group(const DevOutputs& O, DevControl* ctl,
 }
 
 // How many rays a launch is for, which sets its register budget: many (a full
-// wave of lanes several times over), few per lane, or (full Dormand-Prince only)
-// so few that one ray's chain is the time -- then its stages are unrolled.
+// wave of lanes several times over), few per lane, or so few that one ray's
+// chain is the time -- then its stages are unrolled.
 enum : int { kSizeLarge = 0, kSizeSmall = 1, kSizeChain = 2 };
 
 // Band passes of at most this many rays take the unrolled form: about a ray a
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kTraceBlock,
       else if (GROUP)
         res = attempt_fp64_group<METRIC>(PL, R, role, k1, k1_valid, acc, h_used);
       else
-        res = attempt_fp64<METRIC>(PL, R, K, k1_valid, acc, h_used);
+        res = attempt_fp64<METRIC, SIZE == kSizeChain>(PL, R, K, k1_valid, acc, h_used);
       n_att += 1;
       if (acc) n_acc += 1;
       int done_cls = -1;
@@ -602,16 +602,13 @@ const void* select_group(const DevParams& P) {
 }
 
 // Renders of so few samples are traced by the group kernel from the camera:
-// there each lane of the other kernel has at most one ray, and the time is one ray's
-// chain.  Lane per ray / group, ms: Schwarzschild with a thin disk at 32x24
-// 0.97 / 0.48, 128^2 1.53 / 1.02, 160^2 1.56 / 1.43, 200^2 1.93 / 1.88, 256^2
-// 1.92 / 2.76; Kerr without a disk at 64^2 1.96 / 1.36, 160^2 3.67 / 3.44, 200^2
-// 3.67 / 4.08.  So the line is at 2^15 samples.
-#ifndef GG_GROUP_MAX_RAYS
-#define GG_GROUP_MAX_RAYS 32768
-#endif
+// there each lane of the other kernels has at most one ray, and the time is one ray's
+// chain.  Lane per ray (unrolled) / group, ms: Schwarzschild with a thin disk at 64^2 0.93 /
+// 0.65, 100^2 1.12 / 0.81, 128^2 1.14 / 1.04, 165^2 1.39 / 1.54, 200^2 1.52 / 1.88; Kerr without
+// a disk 64^2 1.61 / 1.39, 128^2 1.79 / 1.96, 180^2 2.78 / 3.38.
+constexpr uint64_t kGroupRays = 1ull << 14;
 bool group_render(const DevParams& P) {
-  return P.stepper == kStepperReference && !P.attempt_budget && P.n_rays <= GG_GROUP_MAX_RAYS;
+  return P.stepper == kStepperReference && !P.attempt_budget && P.n_rays <= kGroupRays;
 }
 
 // Kerr camera passes of fewer samples than this run the 4-CTA budget of the
@@ -641,24 +638,37 @@ const void* select_metric(const DevParams& P) {
   return select_disk<kMetricSchwarzschild, STEPPER, kSizeLarge>(P);
 }
 
+template <int STEPPER>
+const void* select_chain(const DevParams& P) {
+  return P.metric == kMetricKerr ? select_disk<kMetricKerr, STEPPER, kSizeChain>(P)
+                                 : select_disk<kMetricSchwarzschild, STEPPER, kSizeChain>(P);
+}
+
 // Full Dormand-Prince camera passes of at most this many samples take the
 // unrolled form.  Rolled / unrolled, ms, the differentiable forward: 64^2 1.83 /
 // 1.52, 128^2 2.84 / 2.32, 160^2 2.26 / 1.98, 200^2 2.53 / 2.34, 230^2 2.90 /
 // 2.65, 256^2 3.16 / 3.39, 512^2 7.2 / 8.5.
 constexpr uint64_t kChainRays = 3ull << 14;
+// The reference's step: up to 2^18, 2^17 with the volumetric disk, whose work at
+// every step wants more warps.  Rolled / unrolled, ms: Schwarzschild with a thin disk
+// at 200^2 1.90 / 1.52, 256^2 1.97 / 1.66, 400^2 3.16 / 2.69, 500^2 3.91 / 3.65, 700^2 5.75 /
+// 5.87; Kerr without a disk 200^2 3.66 / 3.37, 320^2 7.0 / 6.6, 500^2 10.99 / 11.00; with the
+// volumetric disk 200^2 4.72 / 4.39, 320^2 9.08 / 9.01, 450^2 14.2 / 15.4.
+constexpr uint64_t kChainRaysReference = 1ull << 18, kChainRaysVolumetric = 1ull << 17;
 const void* select_trace(const DevParams& P) {
   if (group_render(P)) return select_group(P);
-  const bool chain = P.stepper == kStepperDP45 && P.n_rays <= kChainRays;
+  const bool full = P.stepper == kStepperDP45;
+  const bool chain = P.n_rays <= (full                        ? kChainRays
+                                  : P.disk == kDiskVolumetric ? kChainRaysVolumetric
+                                                              : kChainRaysReference);
   // gg_forward_ckpt admits only Kerr, the thin disk and the full stepper
   if (P.ckpt)
     return chain ? trace_fn<kMetricKerr, kDiskThin, kStepperDP45, kSrcCamera, false, false, true,
                             kSizeChain>()
                  : trace_fn<kMetricKerr, kDiskThin, kStepperDP45, kSrcCamera, false, false, true>();
   if (chain)
-    return P.metric == kMetricKerr ? select_disk<kMetricKerr, kStepperDP45, kSizeChain>(P)
-                                   : select_disk<kMetricSchwarzschild, kStepperDP45, kSizeChain>(P);
-  return P.stepper == kStepperDP45 ? select_metric<kStepperDP45>(P)
-                                   : select_metric<kStepperReference>(P);
+    return full ? select_chain<kStepperDP45>(P) : select_chain<kStepperReference>(P);
+  return full ? select_metric<kStepperDP45>(P) : select_metric<kStepperReference>(P);
 }
 
 // The FP64 pass of the mixed form: full Dormand-Prince, thin disk or none.

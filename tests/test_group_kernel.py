@@ -1,8 +1,8 @@
-"""The group kernel (several lanes per ray) against the lane-per-ray kernel.
+"""The group kernel (several lanes per ray) against the lane-per-ray kernels.
 
 Renders of the reference's step with few samples run on the group kernel, and
-larger ones hand their last rays to it; renders with an attempt budget never
-do.  Both carry out the same operations in the same order per ray, so every
+larger ones, by their size on a kernel with its stages unrolled or in a loop,
+hand their last rays to it; renders with an attempt budget never do.  Both carry out the same operations in the same order per ray, so every
 output has to agree bit for bit: one sample, sizes that leave a group or a
 warp part empty, both sides of the size rule, and images large enough to
 drain into the second pass, over the metrics, disks, scenes, error norms and
@@ -31,8 +31,14 @@ CASES = [
     (31, 17, 2, True, "volumetric", False, 0.0),
     (29, 23, 1, False, "volumetric", True, 0.0),
     (47, 31, 1, True, "none", True, 0.0),
-    (256, 128, 1, False, "none", False, 0.0),   # the size rule's last group render
-    (257, 128, 1, True, "none", False, 0.0),    # and the first that drains into it
+    (128, 128, 1, False, "none", False, 0.0),   # the size rule's last group render
+    (129, 128, 1, True, "none", False, 0.0),    # and the first that drains into it
+    (256, 128, 1, False, "none", False, 0.0),
+    (257, 128, 1, True, "none", False, 0.0),
+    (512, 512, 1, False, "thin", False, 1e-8),  # the last unrolled render
+    (513, 512, 1, True, "none", False, 1e-8),   # and the first rolled one
+    (512, 256, 1, True, "volumetric", False, 0.0),
+    (513, 256, 1, False, "volumetric", True, 0.0),
     (301, 200, 1, False, "volumetric", False, 0.0),
     (301, 200, 1, True, "thin", False, 1e-8),
     (201, 100, 2, True, "volumetric", True, 0.0),
