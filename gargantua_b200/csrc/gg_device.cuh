@@ -598,7 +598,7 @@ GG_DEV bool end_attempt_fp64(const DevParams& P, Ray& R, const double nv[4], con
 // Returns the StepResult; `accepted` and `h_used` describe an advance.
 template <int METRIC, bool UNROLL>
 //
-// UNROLL: see attempt_dp45_fp64.
+// UNROLL: kStageUnrolled of attempt_dp45_fp64, else kStageArms.
 // `k1_valid` says K(0, .) already holds a(x, v) for the current state: the
 // reference's k7 is evaluated at (pos + h vel, new_vel), exactly the state an
 // accepted step moves to, so it is the next attempt's k1 (first same as
@@ -916,6 +916,29 @@ GG_DEV void stage_state(const Ray& R, double h, double hh, const KS& K, double p
   }
 }
 
+// The same sums as one loop over the earlier stages.
+template <class KS>
+GG_DEV void stage_state_looped(int S, const Ray& R, double h, double hh, const KS& K, double px[4],
+                               double pw[4]) {
+  const double ha = h * kDP.A[S];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    px[i] = fma(ha, R.v[i], R.x[i]);
+    pw[i] = R.v[i];
+  }
+#pragma unroll 1
+  for (int l = 0; l < S; ++l) {
+    double k[4];
+    K.get(l, k);
+    const double cv = h * kDP.B[S][l], cb = hh * kDP.Abar[S][l];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      pw[i] = fma(cv, k[i], pw[i]);
+      px[i] = fma(cb, k[i], px[i]);
+    }
+  }
+}
+
 // ex += sum_l Ebar_l k_l, ev += sum_l E_l k_l over the seven stages, in order.
 template <int L, class KS>
 GG_DEV void error_sums_fp64(const KS& K, double ex[4], double ev[4]) {
@@ -953,11 +976,17 @@ GG_DEV bool dp45_stage(const DevParams& P, const Ray& R, double h, double hh, co
 // One full Dormand-Prince attempt in FP64.  Same contract as attempt_fp64;
 // with k1_valid the previous step's last stage (K(6, .), evaluated at the
 // accepted state) is copied to K(0, .) first.  KS is where the stage
-// derivatives live.  UNROLL: the seven stages one after the other instead of
-// a loop over one copy of the right-hand side.  That code is too long for the
-// instruction cache of a full SM, but a warp alone on its scheduler runs it
-// with fewer moves and branches: 2.3 against 2.8 ms on the 128^2 forward.
-template <int METRIC, bool UNROLL = false, class KS>
+// derivatives live.  CODE: how much code an attempt is.  The right-hand side
+// in a loop over the stages, the stages' sums unrolled in arms of a switch
+// (kStageArms); those sums in a loop too (kStageLooped), for the band passes of
+// many rays, whose warps are all at different places and wait for
+// instructions (1.2 to 1.9 cycles per issue): the near view at 2048^2 x 4 takes
+// 83.2 ms with arms and 81.9 looped, the 64-scene batch 83.9 and 82.4; or
+// everything unrolled (kStageUnrolled), too long for a full SM, but a warp
+// alone on its scheduler runs it with fewer moves and branches: 2.3 against
+// 2.8 ms on the 128^2 forward.
+enum StageCode : int { kStageArms, kStageLooped, kStageUnrolled };
+template <int METRIC, StageCode CODE = kStageArms, class KS>
 GG_DEV int attempt_dp45_fp64(const DevParams& P, Ray& R, const KS& K, bool& k1_valid,
                              bool& k7_pending, bool& accepted, double& h_used, StepEnd& end) {
   accepted = false;
@@ -972,7 +1001,7 @@ GG_DEV int attempt_dp45_fp64(const DevParams& P, Ray& R, const KS& K, bool& k1_v
   const double h = R.h, hh = h * h;
   double xn[4], vn[4];
   const int s_first = __any_sync(__activemask(), !k1_valid) ? 0 : 1;
-  if (UNROLL) {
+  if (CODE == kStageUnrolled) {
     if (s_first == 0) {
       Geometry<METRIC, kStepperDP45> G;
       G.at(P, R.x[1], R.x[2]);
@@ -994,28 +1023,37 @@ GG_DEV int attempt_dp45_fp64(const DevParams& P, Ray& R, const KS& K, bool& k1_v
 #pragma unroll 1
   for (int s = s_first; s < 7; ++s) {
     double px[4], pw[4], a[4];
-    switch (s) {  // the last pass leaves the step's end in (px, pw)
-      case 0:
+    // the last pass leaves the step's end in (px, pw)
+    auto step_end = [&]() {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          px[i] = R.x[i];
-          pw[i] = R.v[i];
-        }
-        break;
-      case 1: stage_state<1>(R, h, hh, K, px, pw); break;
-      case 2: stage_state<2>(R, h, hh, K, px, pw); break;
-      case 3: stage_state<3>(R, h, hh, K, px, pw); break;
-      case 4: stage_state<4>(R, h, hh, K, px, pw); break;
-      case 5: stage_state<5>(R, h, hh, K, px, pw); break;
-      default:
-        stage_state<6>(R, h, hh, K, px, pw);
+      for (int i = 0; i < 4; ++i) {
+        xn[i] = px[i];
+        vn[i] = pw[i];
+      }
+      if (!(isfinite(px[0]) && isfinite(px[3]))) px[1] = -1.0;
+    };
+    if (CODE == kStageLooped) {
+      stage_state_looped(s, R, h, hh, K, px, pw);
+      if (s == 6) step_end();
+    } else {
+      switch (s) {
+        case 0:
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          xn[i] = px[i];
-          vn[i] = pw[i];
-        }
-        if (!(isfinite(px[0]) && isfinite(px[3]))) px[1] = -1.0;
-        break;
+          for (int i = 0; i < 4; ++i) {
+            px[i] = R.x[i];
+            pw[i] = R.v[i];
+          }
+          break;
+        case 1: stage_state<1>(R, h, hh, K, px, pw); break;
+        case 2: stage_state<2>(R, h, hh, K, px, pw); break;
+        case 3: stage_state<3>(R, h, hh, K, px, pw); break;
+        case 4: stage_state<4>(R, h, hh, K, px, pw); break;
+        case 5: stage_state<5>(R, h, hh, K, px, pw); break;
+        default:
+          stage_state<6>(R, h, hh, K, px, pw);
+          step_end();
+          break;
+      }
     }
     // is_valid_position; t and phi overflow only with a stage derivative that is not
     // finite, which reaches r by the next stage, so they are tested at the last

@@ -304,7 +304,9 @@ __global__ void __launch_bounds__(kTraceBlock,
       StepEnd end;
       int res;
       if (STEPPER == kStepperDP45)
-        res = attempt_dp45_fp64<METRIC, SIZE == kSizeChain>(
+        res = attempt_dp45_fp64<METRIC, SIZE == kSizeChain    ? kStageUnrolled
+                                        : SRC == kSrcQueue ? kStageLooped
+                                                           : kStageArms>(
             PL, R, K, k1_valid, k7_pending, acc, h_used, end);
       else if (GROUP)
         res = attempt_fp64_group<METRIC>(PL, R, role, k1, k1_valid, acc, h_used);
