@@ -93,6 +93,7 @@ struct gg_ctx {
   void* scene_nodes = nullptr;
   size_t scene_nodes_cap = 0;
   bool scene_set = false;
+  float scene_lo[3] = {0, 0, 0}, scene_hi[3] = {0, 0, 0};  // its box, widened
   bool pending = false;            // stats of the last device-pointer render not read yet
   gg_stats_t last{};
   std::mutex mu;
@@ -392,6 +393,8 @@ void build_params(const gg_metric_t* metric, const gg_camera_t* camera, const gg
     P.density_0 = disk->density_0;
     P.temperature_0 = disk->temperature_0;
     P.emissivity_index = disk->emissivity_index;
+    // exp(-z^2 / 2 H^2) is 0 from |z| = 38.7 H on (the smallest double is e^-744.4)
+    P.r_clear = std::hypot(disk->r_outer, 39.0 * disk->scale_height) * (1.0 + 1e-9);
   }
   P.sky = opts->sky;
   P.sky_rows = opts->sky_rows;
@@ -411,6 +414,10 @@ int attach_sky_map(const gg_ctx* c, DevParams* P) {
     if (!c->scene_set) return GG_ERR_INVALID_ARG;
     P->prims = static_cast<const gg::ScenePrim*>(c->scene_prims);
     P->nodes = static_cast<const gg::SceneNode*>(c->scene_nodes);
+    for (int i = 0; i < 3; ++i) {
+      P->scene_lo[i] = c->scene_lo[i];
+      P->scene_hi[i] = c->scene_hi[i];
+    }
   }
   if (P->sky != gg::kSkyHdri) return GG_OK;
   if (!c->hdri) return GG_ERR_INVALID_ARG;
@@ -1138,6 +1145,13 @@ GG_API int gg_set_scene(gg_ctx* c, const gg_prim_t* prims, uint32_t n) {
           cudaSuccess ||
       cudaStreamSynchronize(c->stream) != cudaSuccess)
     return GG_ERR_CUDA;
+  // widened by 1e-4 of the coordinate's size and of 1 (M): the FP32 rounding of
+  // a position at the box is a thousandth of that, the hit tests' less
+  for (int i = 0; i < 3; ++i) {
+    const double lo = nodes[0].lo[i], hi = nodes[0].hi[i];
+    c->scene_lo[i] = (float)(lo - 1e-4 * (1.0 + std::fabs(lo)));
+    c->scene_hi[i] = (float)(hi + 1e-4 * (1.0 + std::fabs(hi)));
+  }
   c->scene_set = true;
   return GG_OK;
 }

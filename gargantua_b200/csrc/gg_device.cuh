@@ -314,14 +314,13 @@ struct Gmet {
   double tt, phph, tph;
 };
 
+// s, c: sine and cosine of the polar angle.
 template <int METRIC>
-GG_DEV Gmet metric_tensor(const DevParams& P, double r_in, double th) {
+GG_DEV Gmet metric_tensor(const DevParams& P, double r_in, double s, double c) {
   const double r = fmax(r_in, 1e-10);
-  const double s = sin(th);
   Gmet g;
   if (METRIC == kMetricKerr) {  // kerr.rs:61-94
     const double m = P.mass, a = P.spin, a2 = a * a;
-    const double c = cos(th);
     const double sig = fma(r, r, mul_rn(a2 * c, c));
     const double sin2 = s * s;
     g.tt = -sub_rn(1.0, 2.0 * m * r / sig);
@@ -339,8 +338,9 @@ GG_DEV Gmet metric_tensor(const DevParams& P, double r_in, double th) {
 // metric's orbital_four_velocity (schwarzschild.rs:146-153, kerr.rs:439-449)
 // and circular_orbit_velocity (metric.rs:82-94).
 template <int METRIC>
-GG_DEV double redshift_factor(const DevParams& P, double r, double th, const double p[4]) {
-  const Gmet g = metric_tensor<METRIC>(P, r, th);
+GG_DEV double redshift_factor(const DevParams& P, double r, double s, double c,
+                              const double p[4]) {
+  const Gmet g = metric_tensor<METRIC>(P, r, s, c);
   const double p_t = fma(g.tph, p[3], mul_rn(g.tt, p[0]));
   const double e_obs = fmax(-p_t / P.sqrt_neg_gtt_obs, 0.0);
   bool has_orbit;
@@ -373,6 +373,11 @@ GG_DEV double redshift_factor(const DevParams& P, double r, double th, const dou
     e_emit = fmax(g_tt_emit > 0.0 ? -p_t / sqrt(g_tt_emit) : 0.0, 0.0);
   }
   return e_emit > 0.0 ? e_obs / e_emit : 0.0;
+}
+
+template <int METRIC>
+GG_DEV double redshift_factor(const DevParams& P, double r, double th, const double p[4]) {
+  return redshift_factor<METRIC>(P, r, sin(th), cos(th), p);
 }
 
 // ---------------------------------------------------------------------------

@@ -101,6 +101,7 @@ struct DevParams {
   int disk;
   int pad1;
   double r_inner, r_outer, scale_height, density_0, temperature_0, emissivity_index;
+  double r_clear;  // volumetric: beyond this radius the disk's density is 0 everywhere
   // sky
   int sky;
   uint32_t sky_rows, sky_cols;
@@ -115,6 +116,7 @@ struct DevParams {
   const ScenePrim* prims;
   const SceneNode* nodes;
   uint32_t scene;
+  float scene_lo[3], scene_hi[3];  // the scene's box, widened (near_scene)
   // gg_forward_ckpt: the FP64 kernel also stores each ray's checkpoints and
   // DiffRay (DevOutputs::ckpt, diff_rays)
   uint32_t ckpt;

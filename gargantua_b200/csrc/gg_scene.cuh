@@ -82,6 +82,20 @@ GG_DEV bool quad_hit(const ScenePrim& Q, const double o[3], const double d[3], d
   return true;
 }
 
+// Whether the chord from a to b may meet the scene at all: their boxes overlap,
+// the scene's widened (DevParams::scene_lo) by far more than the hit tests
+// round.  Most steps of a picture are nowhere near the objects; this spares
+// them the walk's reciprocals and its first node.
+GG_DEV bool near_scene(const DevParams& P, const double a[3], const double b[3]) {
+  bool near = true;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const float x = (float)a[i], y = (float)b[i];
+    near = near && fmaxf(x, y) >= P.scene_lo[i] && fminf(x, y) <= P.scene_hi[i];
+  }
+  return near;
+}
+
 // Nearest hit of the chord o + t d, t in (0, 1), over the hierarchy
 // (BvhNode::hit, accel/bvh.rs:184-254: t_max shrinks to each hit found).
 // Returns the primitive index or -1.
@@ -155,7 +169,7 @@ GG_DEV void scene_shade(const DevParams& P, int k, double t, const double o[3], 
   // cartesian_to_spherical (tracer.rs:20-28) of the hit point, then g^4
   const double r = fmax(__dsqrt_rn(dot3_nc(point, point)), 1e-10);
   const double th = acos(fmin(fmax(__ddiv_rn(point[2], r), -1.0), 1.0));
-  const Gmet g = metric_tensor<METRIC>(P, r, th);
+  const Gmet g = metric_tensor<METRIC>(P, r, sin(th), cos(th));
   const double g_tt_emit = -g.tt, g_tt_obs = -P.cam_g_tt;
   double g4 = 0.0;
   if (!(g_tt_emit <= 0.0 || g_tt_obs <= 0.0)) {

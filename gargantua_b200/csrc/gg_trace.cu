@@ -127,6 +127,9 @@ __global__ void __launch_bounds__(kTraceBlock,
   __shared__ BlockStats bs;
   __shared__ double2 k_smem[GROUP ? 1 : 7][2][kTraceBlock];  // stage derivatives, see KStore
   const KStore K{k_smem};
+  // SCENE: the Cartesian image of the current position, if cart_valid
+  __shared__ double cart_smem[SCENE ? 3 : 1][kTraceBlock];
+  bool cart_valid = false;
   GroupRole role;
   double k1[4];  // GROUP: a(x, v) of the current state if k1_valid
   if (GROUP) role = GroupRole::at(lane);
@@ -214,6 +217,7 @@ __global__ void __launch_bounds__(kTraceBlock,
         crossed = false;
         k1_valid = false;
         k7_pending = false;
+        cart_valid = false;
         if (from_chain) {
           const ChainRay& q = O.chain[wbase + rank];
 #pragma unroll
@@ -327,11 +331,19 @@ __global__ void __launch_bounds__(kTraceBlock,
         // trace_ray_with_scene (tracer.rs:218-236): the chord between the
         // step's ends, in Cartesian coordinates, against the scene
         double cb[3], ca[3], dd[3];
-        sph_to_cart(xb, cb);
+        if (cart_valid) {  // the last step's end
+#pragma unroll
+          for (int i = 0; i < 3; ++i) cb[i] = cart_smem[i][threadIdx.x];
+        } else {
+          sph_to_cart(xb, cb);
+        }
         sph_to_cart(R.x, ca);
 #pragma unroll
+        for (int i = 0; i < 3; ++i) cart_smem[i][threadIdx.x] = ca[i];
+        cart_valid = true;
+#pragma unroll
         for (int i = 0; i < 3; ++i) dd[i] = sub_rn(ca[i], cb[i]);
-        if (dot3_nc(dd, dd) > 0.0) {
+        if (near_scene(PL, cb, ca) && dot3_nc(dd, dd) > 0.0) {
           double t_hit;
           const int k = scene_nearest(PL, cb, dd, t_hit);
           if (k >= 0) {
@@ -438,10 +450,16 @@ __global__ void __launch_bounds__(kTraceBlock,
       if (DISK == kDiskVolumetric && done_cls < 0) {
         // trace_ray_with_disk (tracer.rs:96-145)
         const double dlambda = fmax(R.lam - lam_b, 0.0);
-        if (dlambda > 0.0) {
-          double mid[4];
+        double mid[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) mid[i] = 0.5 * (xb[i] + R.x[i]);
+        for (int i = 0; i < 4; ++i) mid[i] = 0.5 * (xb[i] + R.x[i]);
+        // Inside r_inner the distance from the axis is too, and beyond r_clear
+        // either it is past r_outer or the density underflows to 0: most steps of
+        // a picture need no sine here.  With this, the sine and cosine shared
+        // with the redshift and (SCENE) each position's Cartesian image kept
+        // for the next step: the command line's disk at 800x600 12.7 -> 12.1 ms,
+        // the lensed spheres with the disk 26.3 -> 23.0.
+        if (dlambda > 0.0 && mid[1] >= PL.r_inner && mid[1] <= PL.r_clear) {
           double sn, cs;
           sincos(mid[2], &sn, &cs);
           const double cap_r = mid[1] * fabs(sn);
@@ -455,7 +473,7 @@ __global__ void __launch_bounds__(kTraceBlock,
               double pm[4];
 #pragma unroll
               for (int i = 0; i < 4; ++i) pm[i] = 0.5 * (vb[i] + R.v[i]);
-              const double g = redshift_factor<METRIC>(PL, mid[1], mid[2], pm);
+              const double g = redshift_factor<METRIC>(PL, mid[1], sn, cs, pm);
               const double g2 = g * g;
               inten = inten + j * (g2 * g2) * dlambda * trans;
               trans = trans * exp(-rho * dlambda * 0.1);
