@@ -73,6 +73,8 @@ __device__ __noinline__ bool hand_to_group(const DevOutputs& O, DevControl* ctl,
   return true;
 }
 
+constexpr int kPendSky = 0x100;  // see `pend`
+
 // How many rays a launch is for, which sets its register budget: many (a full
 // wave of lanes several times over), few per lane, or so few that one ray's
 // chain is the time -- then its stages are unrolled.
@@ -136,14 +138,6 @@ __global__ void __launch_bounds__(kTraceBlock,
   if (threadIdx.x < sizeof(BlockStats) / 8)
     reinterpret_cast<unsigned long long*>(&bs)[threadIdx.x] = 0ull;
   __syncthreads();
-  auto finish = [&](const DevParams& pp, const DevOutputs& oo, uint64_t i, int cls, const Ray& r,
-                    uint32_t na, uint32_t nc, double inten_o, double temp_o, bool cr,
-                    double sky_th, double sky_ph) {
-    finish_sample(pp, oo, i, cls, r, na, nc, inten_o, temp_o, cr, sky_th, sky_ph);
-    atomicAdd(&bs.attempts, (unsigned long long)na);
-    atomicAdd(&bs.accepted, (unsigned long long)nc);
-    atomicAdd(&bs.cls[cls], 1ull);
-  };
   uint32_t n_att0 = 0;  // kSrcQueue: attempts the ray had made before the hand-off
 
   Ray R;
@@ -155,6 +149,14 @@ __global__ void __launch_bounds__(kTraceBlock,
   bool crossed = false;
   bool k1_valid = false;    // K(0, .) holds a(x, v) of the current state
   bool k7_pending = false;  // full DP: K(6, .) is the next k1, copy pending
+  // A ray that ends is finished at the next refill, by every lane of the warp that
+  // has one: its redshift, shading and encoding are nine pow() and as many
+  // divisions, more than an attempt, and ran a lane at a time where the ray ended.
+  // The class, with kPendSky if (inten, trans) hold where the sky is read.
+  // Measured before / after, ms: Schwarzschild disk at 800x600 12.1 / 10.9, near view
+  // at 1024^2 9.9 / 9.0, 256^2 thin disk 1.63 / 1.52, 1080p full Dormand-Prince 42.2 /
+  // 40.2, the 512^2 forward 7.3 / 6.9, the 1080p drop-in frame 35.1 / 35.0.
+  int pend = -1;
   uint32_t n_ckpt = 0;      // CKPT: checkpoints of the ray so far
   auto save_ckpt = [&]() {
     if (n_ckpt < O.ckpt_per_ray) {
@@ -177,6 +179,44 @@ __global__ void __launch_bounds__(kTraceBlock,
       STEPPER == kStepperReference && SRC == kSrcCamera && !GROUP && !CKPT && !BATCH;
 
   for (;;) {
+    // ---- finish the rays that ended ---------------------------------------
+    if (pend >= 0) {
+      const DevParams& PL = BATCH ? B.scenes[scene].P : P;
+      const DevOutputs& OL = BATCH ? B.scenes[scene].O : O;
+      const int cls = pend & ~kPendSky;
+      if (writer) {
+        if (SCENE && cls == kClsScene) {
+          const double rgb[3] = {cart_smem[0][threadIdx.x], cart_smem[SCENE ? 1 : 0][threadIdx.x],
+                                 cart_smem[SCENE ? 2 : 0][threadIdx.x]};
+          finish_scene_sample(PL, OL, idx, R, n_att, n_acc, inten, rgb);
+        } else {
+          double out_int = 0.0, out_temp = 0.0, sky_th = R.x[2], sky_ph = R.x[3];
+          if (pend & kPendSky) {
+            sky_th = inten;
+            sky_ph = trans;
+          }
+          if (DISK == kDiskThin && cls == kClsDisk) {
+            const double g = redshift_factor<METRIC>(PL, R.x[1], kHalfPi, R.v);
+            const double q = PL.r_inner / R.x[1];
+            const double g2 = g * g;
+            out_int = (g2 * g2) * pow(q, PL.emissivity_index);
+            out_temp = g * pow(q, 0.75);
+          } else if (cls == kClsDisk) {
+            out_int = inten;
+            out_temp = PL.temperature_0;
+          }
+          finish_sample(PL, OL, idx, cls, R, n_att, n_acc, out_int, out_temp, crossed, sky_th,
+                        sky_ph);
+        }
+        atomicAdd(&bs.attempts, (unsigned long long)n_att);
+        atomicAdd(&bs.accepted, (unsigned long long)n_acc);
+        atomicAdd(&bs.cls[cls], 1ull);
+        if (SRC == kSrcQueue) atomicAdd(&bs.fp64_att, (unsigned long long)(n_att - n_att0));
+      }
+      if (CKPT) O.diff_rays[idx] = DiffRay{n_acc, n_ckpt, cls, 0u};
+      pend = -1;
+    }
+
     // ---- refill lanes whose ray finished ----------------------------------
     unsigned need = __ballot_sync(kFull, !live);
     if (P.attempt_budget && need && !wdone) {
@@ -319,7 +359,6 @@ __global__ void __launch_bounds__(kTraceBlock,
       n_att += 1;
       if (acc) n_acc += 1;
       int done_cls = -1;
-      double out_int = 0.0, out_temp = 0.0;
       // full Dormand-Prince, checkerboard sky, thin disk or none: the sky is
       // read where the ray meets the escape sphere (sky_at_cross)
       constexpr bool kSkyCross = STEPPER == kStepperDP45 && DISK != kDiskVolumetric;
@@ -423,11 +462,6 @@ __global__ void __launch_bounds__(kTraceBlock,
             if (r_c >= PL.r_inner && r_c <= PL.r_outer) {
               c[1] = r_c;
               c[2] = kHalfPi;
-              const double g = redshift_factor<METRIC>(PL, r_c, kHalfPi, c + 4);
-              const double q = PL.r_inner / r_c;
-              const double g2 = g * g;
-              out_int = (g2 * g2) * pow(q, PL.emissivity_index);
-              out_temp = g * pow(q, 0.75);
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
                 R.x[i] = c[i];
@@ -479,29 +513,15 @@ __global__ void __launch_bounds__(kTraceBlock,
               trans = trans * exp(-rho * dlambda * 0.1);
               if (trans < 1e-3) {
                 done_cls = kClsDisk;
-                out_int = inten;
-                out_temp = PL.temperature_0;
               }
             }
           }
         }
         if (done_cls < 0 && res != kContinue) {
-          if (inten > 0.0) {
-            done_cls = kClsDisk;
-            out_int = inten;
-            out_temp = PL.temperature_0;
-          } else {
-            done_cls = res == kEscaped ? kClsEscaped : kClsHorizon;
-          }
+          done_cls = inten > 0.0 ? kClsDisk : res == kEscaped ? kClsEscaped : kClsHorizon;
         }
         if (done_cls < 0 && n_att >= PL.max_steps) {
-          if (inten > 0.0) {
-            done_cls = kClsDisk;
-            out_int = inten;
-            out_temp = PL.temperature_0;
-          } else {
-            done_cls = kClsMaxSteps;
-          }
+          done_cls = inten > 0.0 ? kClsDisk : kClsMaxSteps;
         }
       } else if (done_cls < 0) {
         if (res == kHorizon) done_cls = kClsHorizon;
@@ -521,21 +541,17 @@ __global__ void __launch_bounds__(kTraceBlock,
         live = false;
         continue;
       }
-      if (SCENE && done_cls == kClsScene) {
-        if (writer) {
-          finish_scene_sample(PL, OL, idx, R, n_att, n_acc, inten, scene_rgb);
-          atomicAdd(&bs.attempts, (unsigned long long)n_att);
-          atomicAdd(&bs.accepted, (unsigned long long)n_acc);
-          atomicAdd(&bs.cls[kClsScene], 1ull);
+      if (done_cls >= 0) {
+        pend = done_cls;
+        if (SCENE && done_cls == kClsScene) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) cart_smem[c][threadIdx.x] = scene_rgb[c];
         }
-        budget_pending += n_att;
-        live = false;
-      } else if (done_cls >= 0) {
-        if (writer)
-          finish(PL, OL, idx, done_cls, R, n_att, n_acc, out_int, out_temp, crossed,
-               sky_at_cross ? sky_th : R.x[2], sky_at_cross ? sky_ph : R.x[3]);
-        if (CKPT) O.diff_rays[idx] = DiffRay{n_acc, n_ckpt, done_cls, 0u};
-        if (SRC == kSrcQueue) atomicAdd(&bs.fp64_att, (unsigned long long)(n_att - n_att0));
+        if (sky_at_cross && done_cls == kClsEscaped) {
+          pend |= kPendSky;
+          inten = sky_th;
+          trans = sky_ph;
+        }
         budget_pending += n_att;
         live = false;
       }
@@ -553,9 +569,7 @@ __global__ void __launch_bounds__(kTraceBlock,
       if (__shfl_sync(kFull, ab, 0)) {
         wdone = true;
         if (live) {
-          finish(BATCH ? B.scenes[scene].P : P, BATCH ? B.scenes[scene].O : O, idx, kClsBudget,
-                 R, n_att, n_acc, 0.0, 0.0, crossed, R.x[2], R.x[3]);
-          if (SRC == kSrcQueue) atomicAdd(&bs.fp64_att, (unsigned long long)(n_att - n_att0));
+          pend = kClsBudget;
           live = false;
         }
       }
