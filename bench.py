@@ -74,6 +74,19 @@ MIXED_PASS_DRAM_BYTES = 3_325_440 + 43_624_448
 # Renders of this many samples or more run the mixed form's hand-back rounds
 # (kHandBackMinRays in gargantua_b200/csrc/gg_capi.cpp).
 HAND_BACK_MIN_SAMPLES = 1 << 20
+# a band pass whose queue can hold more rays is launched in both of its forms;
+# the one that the queue's length is not for returns at once (gg_trace.cu)
+BAND_CHAIN_RAYS = 1 << 16
+
+
+def mixed_launches(n_samples: int) -> int:
+    """Kernels of one mixed render, per rank: the mixed pass and the FP64 band
+    pass; from 2^20 samples also the round reset, the mixed pass over the rays
+    the band pass hands back and the last FP64 pass."""
+    band = 2 if n_samples > BAND_CHAIN_RAYS else 1
+    return 1 + band + (1 + 1 + band if n_samples >= HAND_BACK_MIN_SAMPLES else 0)
+
+
 FLUSH_BYTES = 256 << 20
 
 
@@ -478,10 +491,7 @@ def run_ours(args) -> None:
         "e2e": {"value": H["samples_per_step"] * steps / e2e_s, "unit": UNIT,
                 "h2d_bytes_per_step": abi.load().gg_struct_size(b"launch_params"),
                 "d2h_bytes_per_step": scene.width * scene.rows * 3},
-        # per step and rank: the mixed kernel and the FP64 band pass; from 2^20
-        # samples per render also the round reset, the mixed pass over the rays
-        # the band pass hands back and the last FP64 pass
-        "gpu_launches": (5 if scene.n_samples >= HAND_BACK_MIN_SAMPLES else 2) * steps,
+        "gpu_launches": mixed_launches(scene.n_samples) * steps,
         "roofline": {"bound": "fp32", "achieved": achieved / 1e12,
                      "peak": peak / 1e12, "unit": "TFLOP/s", "frac": achieved / peak,
                      # DRAM read + write of the FP32 pass, one launch of this frame
@@ -984,7 +994,9 @@ def measure_adjoint(r, steps: int, warmup: int, world: int, rank: int, local: in
                     "h2d_bytes_per_step": abi.load().gg_struct_size(b"launch_params"),
                     "d2h_bytes_per_step": 5 * 8 + 8,
                     "via": "diff.kerr_image (torch.autograd.Function) + loss.backward()"},
-            "gpu_launches": 2 * steps,
+            # the forward; the backward's count, scatter, replay, crossing, chain
+            # and camera kernels (one window of segments at this size)
+            "gpu_launches": 7 * steps,
             "roofline": dict(roofline_entry(attempts // world, fpa, fwd_ms * 1e-3, peaks["fp64"],
                                             "fp64", "trace_fp64_kernel<Kerr, ThinDisk, DP45, "
                                             "camera, CKPT> (the forward; the backward's "
@@ -1149,7 +1161,8 @@ def run_features(args) -> None:
             "cli_png_e2e": {"argv": "gr-renderer --disk (Schwarzschild, 800x600) to a PNG file",
                             "ms": 1e3 * cli_s, "geodesics_per_s": n_cli / cli_s,
                             "png_bytes": png_bytes},
-            "gpu_launches": steps * len(cases)}
+            # the trace and the group pass over what its draining warps hand over
+            "gpu_launches": 2 * steps * len(cases)}
     r.close()
     print(json.dumps(line), flush=True)
 

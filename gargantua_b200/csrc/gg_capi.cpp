@@ -511,9 +511,11 @@ int enqueue(gg_ctx* ctx, const DevParams& P, DevOutputs O, bool want_image,
   O.chain = nullptr;
   O.chain_cap = mixed ? 0u : (uint32_t)gg::chain_capacity(P, (int)grid);
   if (O.chain_cap) {
-    const int st = grow(&ctx->chain, &ctx->chain_cap, sizeof(gg::ChainRay) * O.chain_cap);
-    if (st != GG_OK) return st;
-    O.chain = static_cast<gg::ChainRay*>(ctx->chain);
+    // without the buffer the rays stay in their lanes
+    if (grow(&ctx->chain, &ctx->chain_cap, sizeof(gg::ChainRay) * O.chain_cap) == GG_OK)
+      O.chain = static_cast<gg::ChainRay*>(ctx->chain);
+    else
+      O.chain_cap = 0;
   }
   int rbps = 0;
   if (rounds && (gg::mixed_occupancy(P, &rbps, nullptr, 0, true) != cudaSuccess || rbps < 1))
@@ -1268,18 +1270,23 @@ GG_API int gg_backward(gg_ctx* c, const double* dl_drgb_dev, double grad[5], voi
     st = grow(&c->diff_list, &c->diff_list_cap, sizeof(uint64_t) * plan.entries);
     if (st != GG_OK) return st;
     gg::BackwardWindow w{};
-    uint64_t items = 0;
-    size_t ray_bytes = 0;
-    for (uint64_t e = 0; e < plan.entries; e = w.e1) {
-      w = gg::backward_window(kh + next_bytes, plan, e, gg::kBackwardItems);
-      if (w.g1 - w.g0 > items) items = w.g1 - w.g0;
-      const size_t rb = gg::backward_ray_bytes(w.e1 - w.e0, w.p1 - w.p0);
-      if (rb > ray_bytes) ray_bytes = rb;
+    // windows of 2^18 segments keep 2.1 GB of step records; where the device
+    // cannot give that, smaller ones (2^11: 16 MB)
+    uint64_t most = gg::kBackwardItems;
+    for (;; most >>= 1) {
+      uint64_t items = 0;
+      size_t ray_bytes = 0;
+      for (uint64_t e = 0; e < plan.entries; e = w.e1) {
+        w = gg::backward_window(kh + next_bytes, plan, e, most);
+        if (w.g1 - w.g0 > items) items = w.g1 - w.g0;
+        const size_t rb = gg::backward_ray_bytes(w.e1 - w.e0, w.p1 - w.p0);
+        if (rb > ray_bytes) ray_bytes = rb;
+      }
+      st = grow(&c->diff_rec, &c->diff_rec_cap, gg::backward_rec_bytes(items));
+      if (st == GG_OK) st = grow(&c->diff_ray, &c->diff_ray_cap, ray_bytes);
+      if (st == GG_OK) break;
+      if (most <= (1u << 11)) return st;
     }
-    st = grow(&c->diff_rec, &c->diff_rec_cap, gg::backward_rec_bytes(items));
-    if (st != GG_OK) return st;
-    st = grow(&c->diff_ray, &c->diff_ray_cap, ray_bytes);
-    if (st != GG_OK) return st;
     if (cudaMemcpyAsync(kd, kh, next_bytes + bins_bytes, cudaMemcpyHostToDevice, s) !=
             cudaSuccess ||
         gg::launch_backward_scatter(c->diff_P, D, dl_drgb_dev, reinterpret_cast<uint64_t*>(kd),
@@ -1287,7 +1294,7 @@ GG_API int gg_backward(gg_ctx* c, const double* dl_drgb_dev, double grad[5], voi
                                     s) != cudaSuccess)
       return GG_ERR_CUDA;
     for (uint64_t e = 0; e < plan.entries; e = w.e1) {
-      w = gg::backward_window(kh + next_bytes, plan, e, gg::kBackwardItems);
+      w = gg::backward_window(kh + next_bytes, plan, e, most);
       if (gg::launch_backward_window(
               c->diff_P, D, dl_drgb_dev, static_cast<const uint64_t*>(c->diff_list),
               kd + next_bytes, plan, w, static_cast<double*>(c->diff_rec),

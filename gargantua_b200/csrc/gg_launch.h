@@ -15,14 +15,16 @@ constexpr int kTraceBlock = 128;  // threads per CTA of the trace kernels
 // FP64 band passes, the differentiable render's forward, camera passes of
 // fewer than 2^20 samples -- 4 (128 registers, no spills on the chain);
 // Schwarzschild's lighter right-hand side: 4.
-// Measured on B200 (ms, CTAs 6 / 5 / 4): FP64 drop-in Kerr 1080p 45.3 /
-// 43.8 / 44.8, its full Dormand-Prince form 59.4 / 55.3 / 55.4, the stress
-// frame at 2048^2 x 4 spp 133.5 / 133.6 / 136.2 (drop-in) and 171.7 / 160.4
-// / 161.9 (full DP); band passes, through the mixed 1080p frame 27.0 / 26.7 /
-// 26.3; the 512^2 adjoint's forward 10.1 / 8.9 / 8.6.  At 3 CTAs (168
-// registers) for the band passes and the mixed pass over returned rays, the
-// 1080p frame gains 0.3 ms but the stress frame at 2048^2 x 4 spp, whose band
-// holds 12 % of the attempts, loses 1.3 ms.  The camera passes' budget (5)
+// Measured on B200 (ms, CTAs 6 / 5 / 4 / 3): FP64 drop-in Kerr 1080p 35.4 /
+// 35.1 / 35.9 / 39.5, its full Dormand-Prince form 41.8 / 41.2 / 42.2 / 44.8,
+// a 1024^2 camera close to the hole (drop-in) 10.0 / 9.8 / 9.8 / 10.5.  In an
+// earlier build, whose attempts took a quarter more instructions (6 / 5 / 4):
+// the stress frame at 2048^2 x 4 spp 133.5 / 133.6 / 136.2 (drop-in) and
+// 171.7 / 160.4 / 161.9 (full DP); band passes, through the mixed 1080p frame,
+// 27.0 / 26.7 / 26.3; the 512^2 adjoint's forward 10.1 / 8.9 / 8.6.  At 3 CTAs
+// (168 registers) for that build's band passes and mixed pass over returned
+// rays, the 1080p frame gained 0.3 ms but the 2048^2 x 4 stress frame, whose band
+// holds 12 % of the attempts, lost 1.3 ms.  The camera passes' budget (5)
 // for the band passes of renders from 2^23 samples, whose band holds enough
 // rays to be throughput-bound: 84.9 against 84.2 ms on the stress frame at
 // 2048^2 x 4 spp, 1.291 against 1.285 s at 4096^2 x 16 spp and 2.403 against
