@@ -21,7 +21,7 @@ constexpr unsigned kFull = 0xffffffffu;
 // Kerr frame, FP64 drop-in / mixed ms: period 2: 52.9 / 33.4, 4: 49.9 / 31.1,
 // 8: 47.0 / 29.3, 16: 45.3 / 29.2, 32: 44.3 / 29.4 (fewer ballots and
 // refills; lanes that finish early wait longer).  Measured again for the mixed
-// camera pass at 8 / 16 / 32 (the current build): 1080p 25.6 / 25.7 / 25.9
+// camera pass at 8 / 16 / 32 (a later build): 1080p 25.6 / 25.7 / 25.9
 // ms, the stress view at 2048^2 x 4 spp 83.9 / 82.2 / 84.9 ms, the full stress
 // frame 1.273 / 1.249 / 1.306 s.
 #ifndef GG_TRACE_PERIOD
