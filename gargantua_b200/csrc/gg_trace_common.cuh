@@ -20,10 +20,10 @@ constexpr unsigned kFull = 0xffffffffu;
 // (single-scene renders; batches autotune theirs).  Measured on the 1080p
 // Kerr frame, FP64 drop-in / mixed ms: period 2: 52.9 / 33.4, 4: 49.9 / 31.1,
 // 8: 47.0 / 29.3, 16: 45.3 / 29.2, 32: 44.3 / 29.4 (fewer ballots and
-// refills; lanes that finish early wait longer).  Measured again for the mixed
-// camera pass at 8 / 16 / 32 (a later build): 1080p 25.6 / 25.7 / 25.9
-// ms, the stress view at 2048^2 x 4 spp 83.9 / 82.2 / 84.9 ms, the full stress
-// frame 1.273 / 1.249 / 1.306 s.
+// refills; lanes that finish early wait longer), in an early build.  The mixed
+// camera pass at 16 / 24 / 32 in this one: 1080p 23.7 / 24.0 / 23.8 ms, the
+// stress view at 2048^2 x 4 spp 81.5 / 82.1 / 84.1 ms (8: 2 % more than 16 when
+// last measured).
 #ifndef GG_TRACE_PERIOD
 #define GG_TRACE_PERIOD 32
 #endif
