@@ -71,6 +71,12 @@ __global__ void step_factor_kernel(const double* __restrict__ s2, double* __rest
     out[i] = gg::root10_8_over(s2[i]);
 }
 
+__global__ void rcp_kernel(const float* __restrict__ x, float* __restrict__ out, uint64_t n) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (uint64_t)gridDim.x * blockDim.x)
+    out[i] = gg::rcp(x[i]);
+}
+
 int launch_status() {
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? GG_OK : GG_ERR_CUDA;
@@ -115,5 +121,14 @@ extern "C" GG_API int gg_check_step_factor(const double* s2_dev, double* out_dev
   const uint64_t blocks = (n + 255) / 256;
   step_factor_kernel<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0,
                        static_cast<cudaStream_t>(stream)>>>(s2_dev, out_dev, n);
+  return launch_status();
+}
+
+extern "C" GG_API int gg_check_rcp(const float* x_dev, float* out_dev, uint64_t n, void* stream) {
+  if (n == 0) return GG_OK;
+  if (!x_dev || !out_dev) return GG_ERR_INVALID_ARG;
+  const uint64_t blocks = (n + 255) / 256;
+  rcp_kernel<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0,
+               static_cast<cudaStream_t>(stream)>>>(x_dev, out_dev, n);
   return launch_status();
 }

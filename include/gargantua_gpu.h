@@ -435,6 +435,11 @@ GG_API int gg_check_kerr_vjp(const double* in_dev, double* out_dev, uint64_t n, 
  * stream and return conventions as above. */
 GG_API int gg_check_step_factor(const double* s2_dev, double* out_dev, uint64_t n, void* stream);
 
+/* The reciprocal of the mixed form's FP32 right-hand side and error scales, of
+ * n floats (test use; no reference counterpart).  Same pointer, stream and
+ * return conventions as above. */
+GG_API int gg_check_rcp(const float* x_dev, float* out_dev, uint64_t n, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -247,4 +247,6 @@ extern "C" {
                              stream: *mut c_void) -> c_int;
     pub fn gg_check_step_factor(s2_dev: *const f64, out_dev: *mut f64, n: u64,
                                 stream: *mut c_void) -> c_int;
+    pub fn gg_check_rcp(x_dev: *const f32, out_dev: *mut f32, n: u64,
+                        stream: *mut c_void) -> c_int;
 }
