@@ -761,6 +761,7 @@ BackwardWindow backward_window(const void* bins, const BackwardPlan& plan, uint6
       w.p1 = w.p0;
       begun = true;
     }
+    if (w.e1 > w.e0 && w.g1 - w.g0 >= most) break;  // one ray may have more than `most`
     const uint64_t have = stop - b[k].start - from, left = most - (w.g1 - w.g0);
     uint64_t take = left / b[k].segs;
     if (take > have) take = have;

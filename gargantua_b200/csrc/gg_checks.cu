@@ -9,7 +9,10 @@
 // same directions (and the same velocities for spatial_dir) instead.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <new>
+#include <vector>
 
 #include "../../include/gargantua_gpu.h"
 #include "gg_device.cuh"
@@ -131,4 +134,28 @@ extern "C" GG_API int gg_check_rcp(const float* x_dev, float* out_dev, uint64_t 
   rcp_kernel<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0,
                static_cast<cudaStream_t>(stream)>>>(x_dev, out_dev, n);
   return launch_status();
+}
+
+extern "C" GG_API int gg_check_backward_windows(const uint32_t* counts, uint32_t n_keys,
+                                                uint64_t most, uint64_t* windows, uint64_t cap,
+                                                uint64_t* n) {
+  if (!counts || !n_keys || !most || !windows || !n) return GG_ERR_INVALID_ARG;
+  std::vector<uint64_t> next;
+  std::vector<char> bins;
+  try {
+    next.resize(n_keys);
+    bins.resize(gg::backward_bins_bytes(n_keys));
+  } catch (const std::bad_alloc&) {
+    return GG_ERR_OOM;
+  }
+  const gg::BackwardPlan plan = gg::backward_plan(counts, n_keys, next.data(), bins.data());
+  *n = 0;
+  for (uint64_t e = 0; e < plan.entries && *n < cap; ++*n) {
+    const gg::BackwardWindow w = gg::backward_window(bins.data(), plan, e, most);
+    const uint64_t row[6] = {w.e0, w.e1, w.g0, w.g1, w.p0, w.p1};
+    std::copy(row, row + 6, windows + 6 * *n);
+    if (w.e1 <= e) return GG_ERR_CUDA;  // no progress
+    e = w.e1;
+  }
+  return GG_OK;
 }

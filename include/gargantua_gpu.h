@@ -440,6 +440,14 @@ GG_API int gg_check_step_factor(const double* s2_dev, double* out_dev, uint64_t 
  * return conventions as above. */
 GG_API int gg_check_rcp(const float* x_dev, float* out_dev, uint64_t n, void* stream);
 
+/* The windows in which gg_backward takes an image back, on the host (test use;
+ * no reference counterpart): counts[k] listed rays of n_keys - k segments each,
+ * longest first, at most `most` segments a window (one ray at least).  Writes
+ * up to `cap` rows of 6 (first ray and one past the last, the same in segments
+ * and in segments taken in parallel) and their number. */
+GG_API int gg_check_backward_windows(const uint32_t* counts, uint32_t n_keys, uint64_t most,
+                                     uint64_t* windows, uint64_t cap, uint64_t* n);
+
 #ifdef __cplusplus
 }
 #endif

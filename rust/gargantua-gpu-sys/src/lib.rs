@@ -249,4 +249,6 @@ extern "C" {
                                 stream: *mut c_void) -> c_int;
     pub fn gg_check_rcp(x_dev: *const f32, out_dev: *mut f32, n: u64,
                         stream: *mut c_void) -> c_int;
+    pub fn gg_check_backward_windows(counts: *const u32, n_keys: u32, most: u64,
+                                     windows: *mut u64, cap: u64, n: *mut u64) -> c_int;
 }
