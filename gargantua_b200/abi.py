@@ -175,6 +175,8 @@ _SIGNATURES = {
     "gg_check_rcp": (C.c_int, [C.c_void_p, C.c_void_p, C.c_uint64, C.c_void_p]),
     "gg_check_backward_windows": (C.c_int, [P(C.c_uint32), C.c_uint32, C.c_uint64,
                                             P(C.c_uint64), C.c_uint64, P(C.c_uint64)]),
+    "gg_check_backward_memory": (C.c_int, [C.c_void_p, C.c_uint64, C.c_uint64, P(C.c_uint64),
+                                           P(C.c_uint64)]),
     "gg_render_batch": (C.c_int, [C.c_void_p, P(gg_scene_t), C.c_uint32, P(gg_integrator_t),
                                   P(gg_render_opts_t), C.c_void_p]),
     "gg_render_batch_device": (C.c_int, [C.c_void_p, P(gg_scene_t), C.c_uint32,

@@ -80,6 +80,11 @@ struct gg_ctx {
   size_t diff_rec_cap = 0;
   void* diff_ray = nullptr;
   size_t diff_ray_cap = 0;
+  uint64_t diff_most = gg::kBackwardItems;  // less once an allocation has failed
+  uint64_t diff_windows = 0;                // of the last backward
+  // gg_check_backward_memory: the memory the backward sees, and the largest
+  // allocation of step records that succeeds
+  uint64_t diff_memory = UINT64_MAX, diff_alloc = UINT64_MAX;
   double* diff_grad = nullptr;       // 5 doubles, device
   double* diff_grad_host = nullptr;  // pinned
   // equirectangular sky map (gg_set_hdri), RGB float texels on the device
@@ -443,12 +448,18 @@ int grow_pinned(void** buf, size_t* cap, size_t need) {
   return GG_OK;
 }
 
-int grow(void** buf, size_t* cap, size_t need) {
-  if (need <= *cap) return GG_OK;
+void release(void** buf, size_t* cap) {
   if (*buf) cudaFree(*buf);
   *buf = nullptr;
   *cap = 0;
+}
+
+// At least `need` bytes; a quarter more for the next, up to `full` bytes in all.
+int grow(void** buf, size_t* cap, size_t need, size_t full = SIZE_MAX) {
+  if (need <= *cap) return GG_OK;
+  release(buf, cap);
   size_t want = need + need / 4;
+  if (want > full) want = need > full ? need : full;
   if (cudaMalloc(buf, want) != cudaSuccess) {
     cudaGetLastError();
     if (cudaMalloc(buf, need) != cudaSuccess) {
@@ -460,6 +471,48 @@ int grow(void** buf, size_t* cap, size_t need) {
   }
   *cap = want;
   return GG_OK;
+}
+
+// The step records and per-ray results of the backward's windows: of the
+// largest windows, from kBackwardItems segments down by halves, whose buffers the
+// context has already or which take at most a quarter of what the device has
+// left (the present buffers counted as left).  A device with little left keeps
+// most of it; and a call finds the last one's buffers large enough, rather than
+// giving them back to try for larger ones.  An allocation that fails all the
+// same is tried at half the size, there and from then on.
+int backward_buffers(gg_ctx* c, const void* bins, const gg::BackwardPlan& plan, uint64_t* most) {
+  for (*most = c->diff_most;; *most >>= 1) {
+    const bool least = *most <= gg::kBackwardItemsLeast;
+    uint64_t items = 0, windows = 0;
+    size_t ray_bytes = 0;
+    gg::BackwardWindow w{};
+    for (uint64_t e = 0; e < plan.entries; e = w.e1, ++windows) {
+      w = gg::backward_window(bins, plan, e, *most);
+      if (w.g1 - w.g0 > items) items = w.g1 - w.g0;
+      const size_t rb = gg::backward_ray_bytes(w.e1 - w.e0, w.p1 - w.p0);
+      if (rb > ray_bytes) ray_bytes = rb;
+    }
+    c->diff_windows = windows;
+    const size_t rec_bytes = gg::backward_rec_bytes(items);
+    if (rec_bytes <= c->diff_rec_cap && ray_bytes <= c->diff_ray_cap) return GG_OK;
+    size_t left = 0, total = 0;
+    if (cudaMemGetInfo(&left, &total) != cudaSuccess) return GG_ERR_CUDA;
+    left += c->diff_rec_cap + c->diff_ray_cap;
+    if (left > c->diff_memory) left = c->diff_memory;
+    const size_t share = left / 4, ray_full = ray_bytes + ray_bytes / 4;
+    if (!least && rec_bytes + ray_bytes > share) continue;
+    // what grow adds for the next image stays inside the share too
+    size_t full = gg::backward_rec_bytes(gg::kBackwardItems);
+    if (full + ray_full > share) full = share > ray_full ? share - ray_full : 0;
+    int st = rec_bytes > c->diff_alloc ? GG_ERR_OOM : GG_OK;
+    if (st == GG_OK) st = grow(&c->diff_rec, &c->diff_rec_cap, rec_bytes, full);
+    if (st == GG_OK) st = grow(&c->diff_ray, &c->diff_ray_cap, ray_bytes);
+    if (st == GG_OK) return GG_OK;
+    release(&c->diff_rec, &c->diff_rec_cap);
+    release(&c->diff_ray, &c->diff_ray_cap);
+    c->diff_most = least ? gg::kBackwardItems : *most >> 1;
+    if (least) return st;
+  }
 }
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -1225,6 +1278,17 @@ GG_API int gg_forward_ckpt(gg_ctx* c, const gg_metric_t* metric, double r_cam,
   return GG_OK;
 }
 
+GG_API int gg_check_backward_memory(gg_ctx* c, uint64_t memory, uint64_t largest,
+                                    uint64_t* windows, uint64_t* bytes) {
+  if (!c) return GG_ERR_INVALID_ARG;
+  Lock lock(c);
+  c->diff_memory = memory;
+  c->diff_alloc = largest;
+  if (windows) *windows = c->diff_windows;
+  if (bytes) *bytes = c->diff_rec_cap + c->diff_ray_cap;
+  return GG_OK;
+}
+
 GG_API int gg_backward(gg_ctx* c, const double* dl_drgb_dev, double grad[5], void* stream) {
   if (!c || !dl_drgb_dev || !grad) return GG_ERR_INVALID_ARG;
   Lock lock(c);
@@ -1264,35 +1328,22 @@ GG_API int gg_backward(gg_ctx* c, const double* dl_drgb_dev, double grad[5], voi
                       cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return GG_ERR_CUDA;
+  c->diff_windows = 0;
   const gg::BackwardPlan plan = gg::backward_plan(
       counts, n_keys, reinterpret_cast<uint64_t*>(kh), kh + next_bytes);
   if (plan.entries) {
     st = grow(&c->diff_list, &c->diff_list_cap, sizeof(uint64_t) * plan.entries);
     if (st != GG_OK) return st;
-    gg::BackwardWindow w{};
-    // windows of 2^18 segments keep 2.1 GB of step records; where the device
-    // cannot give that, smaller ones (2^11: 16 MB)
-    uint64_t most = gg::kBackwardItems;
-    for (;; most >>= 1) {
-      uint64_t items = 0;
-      size_t ray_bytes = 0;
-      for (uint64_t e = 0; e < plan.entries; e = w.e1) {
-        w = gg::backward_window(kh + next_bytes, plan, e, most);
-        if (w.g1 - w.g0 > items) items = w.g1 - w.g0;
-        const size_t rb = gg::backward_ray_bytes(w.e1 - w.e0, w.p1 - w.p0);
-        if (rb > ray_bytes) ray_bytes = rb;
-      }
-      st = grow(&c->diff_rec, &c->diff_rec_cap, gg::backward_rec_bytes(items));
-      if (st == GG_OK) st = grow(&c->diff_ray, &c->diff_ray_cap, ray_bytes);
-      if (st == GG_OK) break;
-      if (most <= (1u << 11)) return st;
-    }
+    uint64_t most = 0;
+    st = backward_buffers(c, kh + next_bytes, plan, &most);
+    if (st != GG_OK) return st;
     if (cudaMemcpyAsync(kd, kh, next_bytes + bins_bytes, cudaMemcpyHostToDevice, s) !=
             cudaSuccess ||
         gg::launch_backward_scatter(c->diff_P, D, dl_drgb_dev, reinterpret_cast<uint64_t*>(kd),
                                     static_cast<uint64_t*>(c->diff_list), c->sms,
                                     s) != cudaSuccess)
       return GG_ERR_CUDA;
+    gg::BackwardWindow w{};
     for (uint64_t e = 0; e < plan.entries; e = w.e1) {
       w = gg::backward_window(kh + next_bytes, plan, e, most);
       if (gg::launch_backward_window(

@@ -125,6 +125,7 @@ struct BackwardWindow {
 // Segments of a window: 2.1 GB of step records, one window for most images of
 // 512^2.
 constexpr uint64_t kBackwardItems = 1ull << 18;
+constexpr uint64_t kBackwardItemsLeast = 1ull << 11;  // 16 MB
 cudaError_t launch_backward_count(const DevParams& P, const DiffOut& D, const double* dl_drgb,
                                   uint32_t* bins, int sms, cudaStream_t stream);
 size_t backward_bins_bytes(uint32_t n_keys);

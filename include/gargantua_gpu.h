@@ -448,6 +448,14 @@ GG_API int gg_check_rcp(const float* x_dev, float* out_dev, uint64_t n, void* st
 GG_API int gg_check_backward_windows(const uint32_t* counts, uint32_t n_keys, uint64_t most,
                                      uint64_t* windows, uint64_t cap, uint64_t* n);
 
+/* gg_backward as on a device with little memory left (test use; no reference
+ * counterpart): from now on the context's backward sees at most `memory` bytes
+ * for its buffers, and an allocation of step records of more than `largest`
+ * bytes fails (UINT64_MAX: no such limit).  Writes, when not NULL, the windows of
+ * its last call and the bytes it holds for step records and per-ray results. */
+GG_API int gg_check_backward_memory(gg_ctx* ctx, uint64_t memory, uint64_t largest,
+                                    uint64_t* windows, uint64_t* bytes);
+
 #ifdef __cplusplus
 }
 #endif

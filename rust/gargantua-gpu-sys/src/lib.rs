@@ -251,4 +251,6 @@ extern "C" {
                         stream: *mut c_void) -> c_int;
     pub fn gg_check_backward_windows(counts: *const u32, n_keys: u32, most: u64,
                                      windows: *mut u64, cap: u64, n: *mut u64) -> c_int;
+    pub fn gg_check_backward_memory(ctx: *mut gg_ctx, memory: u64, largest: u64,
+                                    windows: *mut u64, bytes: *mut u64) -> c_int;
 }
