@@ -16,6 +16,7 @@
 
 #include "../../include/gargantua_gpu.h"
 #include "gg_device.cuh"
+#include "gg_host.h"
 #include "gg_mixed.cuh"
 #include "gg_vjp.cuh"
 
@@ -78,6 +79,90 @@ __global__ void rcp_kernel(const float* __restrict__ x, float* __restrict__ out,
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x)
     out[i] = gg::rcp(x[i]);
+}
+
+// `attempts` attempts of every ray of a small frame from the camera, or until it
+// ends: its state and step (x, v, lambda, h), and how many attempts it made, how
+// many were accepted and how many were at max_step.  FORM 0: the reference's
+// step, 1: full Dormand-Prince, 2: that in mixed precision (up to the FP64 band).
+template <int METRIC, int FORM, bool STEADY>
+__global__ void __launch_bounds__(gg::kTraceBlock)
+    steps_kernel(const __grid_constant__ gg::DevParams P, uint32_t attempts, double* state,
+                 uint32_t* counts) {
+  __shared__ double2 k_smem[FORM == 2 ? 1 : 7][2][gg::kTraceBlock];
+  __shared__ __align__(16) char m_smem[FORM == 2 ? gg::mixed_smem_bytes<gg::kTraceBlock>() : 16];
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= P.n_rays) return;
+  gg::Ray R;
+  double u, v;
+  gg::sample_uv(P, i, u, v);
+  gg::init_ray(P, u, v, R);
+  bool k1_valid = false, k7_pending = false, acc = false;
+  uint32_t n_att = 0, n_acc = 0, n_max = 0;
+  if constexpr (FORM == 2) {
+    const gg::MixedSmem K = gg::MixedSmem::at(m_smem);
+    gg::MixedRegs S;
+    gg::mixed_load(R, i, K, S);
+    for (; n_att < attempts; ++n_att) {
+      const float r = K.comp(gg::kSlotXh, 1), th = K.comp(gg::kSlotXh, 2);
+      if (r < P.band_r || th < P.pole_band || th > gg::kPiHi - P.pole_band) break;
+      n_max += S.h == P.max_step;
+      float hf = 0.0f;
+      if (gg::attempt_dp45_mixed<METRIC, STEADY>(P, S, K, k1_valid, k7_pending, acc, hf) !=
+          gg::kContinue)
+        break;
+      const float th_a = th + K.comp(gg::kSlotDx, 2);
+      if (acc && !(th_a > 0.0f && th_a < gg::kPiHi)) break;
+      if (acc) gg::mixed_advance(S, K, hf, k1_valid, k7_pending);
+      n_acc += acc;
+    }
+    R = gg::mixed_fp64(K, S);
+  } else {
+    const gg::KStore K{k_smem};
+    for (; n_att < attempts; ++n_att) {
+      n_max += R.h == P.max_step;
+      double h_used = 0.0;
+      int res;
+      if constexpr (FORM == 1) {
+        gg::StepEnd end;
+        res = gg::attempt_dp45_fp64<METRIC, gg::kStageArms, STEADY>(P, R, K, k1_valid, k7_pending,
+                                                                    acc, h_used, end);
+      } else {
+        res = gg::attempt_fp64<METRIC, false, STEADY>(P, R, K, k1_valid, acc, h_used);
+      }
+      if (res != gg::kContinue) break;
+      n_acc += acc;
+    }
+  }
+  double* o = state + 10 * i;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    o[c] = R.x[c];
+    o[4 + c] = R.v[c];
+  }
+  o[8] = R.lam;
+  o[9] = R.h;
+  counts[3 * i] = n_att;
+  counts[3 * i + 1] = n_acc;
+  counts[3 * i + 2] = n_max;
+}
+
+template <int METRIC, int FORM>
+void launch_steps(const gg::DevParams& P, bool steady, uint32_t attempts, double* state,
+                  uint32_t* counts, cudaStream_t s) {
+  const unsigned blocks = (unsigned)((P.n_rays + gg::kTraceBlock - 1) / gg::kTraceBlock);
+  if (steady)
+    steps_kernel<METRIC, FORM, true><<<blocks, gg::kTraceBlock, 0, s>>>(P, attempts, state, counts);
+  else
+    steps_kernel<METRIC, FORM, false><<<blocks, gg::kTraceBlock, 0, s>>>(P, attempts, state, counts);
+}
+
+template <int METRIC>
+void launch_steps_form(int form, const gg::DevParams& P, bool steady, uint32_t attempts,
+                       double* state, uint32_t* counts, cudaStream_t s) {
+  if (form == 0) launch_steps<METRIC, 0>(P, steady, attempts, state, counts, s);
+  else if (form == 1) launch_steps<METRIC, 1>(P, steady, attempts, state, counts, s);
+  else launch_steps<METRIC, 2>(P, steady, attempts, state, counts, s);
 }
 
 int launch_status() {
@@ -158,4 +243,25 @@ extern "C" GG_API int gg_check_backward_windows(const uint32_t* counts, uint32_t
     e = w.e1;
   }
   return GG_OK;
+}
+
+extern "C" GG_API int gg_check_steps(const gg_metric_t* metric, const gg_camera_t* camera,
+                                     const gg_integrator_t* integ, uint32_t width,
+                                     uint32_t height, int form, int steady, uint32_t attempts,
+                                     double* state_dev, uint32_t* counts_dev, void* stream) {
+  if (!state_dev || !counts_dev || form < 0 || form > 2) return GG_ERR_INVALID_ARG;
+  gg_render_opts_t opts;
+  gg_render_opts_default(&opts);
+  const int v = gg::validate_render(metric, camera, nullptr, integ, &opts, width, height);
+  if (v != GG_OK) return v;
+  if ((uint64_t)width * height > (1u << 20)) return GG_ERR_INVALID_ARG;
+  gg::DevParams P;
+  gg::make_params(metric, camera, nullptr, integ, &opts, width, height, &P);
+  const cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (P.metric == gg::kMetricKerr)
+    launch_steps_form<gg::kMetricKerr>(form, P, steady != 0, attempts, state_dev, counts_dev, s);
+  else
+    launch_steps_form<gg::kMetricSchwarzschild>(form, P, steady != 0, attempts, state_dev,
+                                                counts_dev, s);
+  return launch_status();
 }

@@ -454,6 +454,7 @@ GG_DEV double fifth_root(double x) {
 // whose steps are mostly below max_step and take the full law).  Measured,
 // before / after: the 1080p Kerr frame 43.9 / 40.6 ms (drop-in) and 55.4 /
 // 50.8 ms (full Dormand-Prince); a 256^2 Schwarzschild render 2.28 / 2.09 ms.
+// (STEADY = false, for gg_check_steps: every attempt takes the full law.)
 constexpr double kSteadyErr = 0.5625;
 
 // Dormand-Prince tableau (geodesic.rs:210-242), in constant memory: a 64-bit
@@ -551,12 +552,13 @@ GG_DEV void stage_velocity(const double v[4], double h, const KS& K, double w[4]
 // The end of a reference attempt: new velocity nv, its embedded error d
 // (geodesic.rs:306-327).  The acceptance test and the step-size law; advances
 // the ray (position not yet normalised) and returns true if the step stands.
+template <bool STEADY = true>
 GG_DEV bool end_attempt_fp64(const DevParams& P, Ray& R, const double nv[4], const double d[4]) {
   const double h = R.h;
   // `steady`: the step is max_step already and every component's error is
   // within kSteadyErr of its scale, so the step is accepted and the law's
   // clamp gives max_step again: the norm's divisions and root are not needed.
-  bool steady = h == P.max_step;
+  bool steady = STEADY && h == P.max_step;
   double sc[4], ssum = 0.0;
   if (P.rtol > 0.0) {
 #pragma unroll
@@ -604,7 +606,6 @@ GG_DEV bool end_attempt_fp64(const DevParams& P, Ray& R, const double nv[4], con
 
 // One call of RK45Integrator::step (geodesic.rs:185-328) in FP64.
 // Returns the StepResult; `accepted` and `h_used` describe an advance.
-template <int METRIC, bool UNROLL>
 //
 // UNROLL: kStageUnrolled of attempt_dp45_fp64, else kStageArms.
 // `k1_valid` says K(0, .) already holds a(x, v) for the current state: the
@@ -613,6 +614,7 @@ template <int METRIC, bool UNROLL>
 // last) unless normalisation reflected theta at a pole; a rejected attempt
 // leaves the state, and so k1, unchanged.  The reference recomputes k1; the
 // values are identical, one right-hand side per attempt cheaper.
+template <int METRIC, bool UNROLL, bool STEADY = true>
 GG_DEV int attempt_fp64(const DevParams& P, Ray& R, const KStore& K, bool& k1_valid,
                         bool& accepted, double& h_used) {
   accepted = false;
@@ -699,7 +701,7 @@ GG_DEV int attempt_fp64(const DevParams& P, Ray& R, const KStore& K, bool& k1_va
     const double ve = combine4(R.v[i], h, K(0, i), K(2, i), K(3, i), K(4, i), k6[i], k7[i]);
     d[i] = sub_rn(nv[i], ve);
   }
-  if (!end_attempt_fp64(P, R, nv, d)) return kContinue;
+  if (!end_attempt_fp64<STEADY>(P, R, nv, d)) return kContinue;
   const bool reflected = R.x[2] < 0.0 || R.x[2] > kPi;
   normalize_coords(R.x);
   if (!reflected) K.set(0, k7);
@@ -994,7 +996,7 @@ GG_DEV bool dp45_stage(const DevParams& P, const Ray& R, double h, double hh, co
 // alone on its scheduler runs it with fewer moves and branches: 2.3 against
 // 2.8 ms on the 128^2 forward.
 enum StageCode : int { kStageArms, kStageLooped, kStageUnrolled };
-template <int METRIC, StageCode CODE = kStageArms, class KS>
+template <int METRIC, StageCode CODE = kStageArms, bool STEADY = true, class KS>
 GG_DEV int attempt_dp45_fp64(const DevParams& P, Ray& R, const KS& K, bool& k1_valid,
                              bool& k7_pending, bool& accepted, double& h_used, StepEnd& end) {
   accepted = false;
@@ -1080,7 +1082,7 @@ GG_DEV int attempt_dp45_fp64(const DevParams& P, Ray& R, const KS& K, bool& k1_v
   error_sums_fp64<0>(K, ex, ev);
   // as in attempt_fp64: an attempt at max_step whose errors are all well
   // inside their scales is accepted and keeps max_step
-  bool steady = h == P.max_step;
+  bool steady = STEADY && h == P.max_step;
   double err = 0.0, tol;
   double s2 = 0.0;
   if (P.rtol > 0.0) {

@@ -529,7 +529,7 @@ GG_DEV bool beyond_max_radius(const DevParams& P, const KS& K) {
 // (mixed_advance applies it).  The horizon test never fires here: the FP64
 // band starts 0.5 M outside the horizon and its buffer.  Invalid stages are
 // judged on r and theta, the coordinates the stages form.
-template <int METRIC, class KS>
+template <int METRIC, bool STEADY = true, class KS>
 GG_DEV int attempt_dp45_mixed(const DevParams& P, MixedRegs& S, const KS& K,
                               bool& k1_valid, bool& k7_pending, bool& accepted, float& hf) {
   accepted = false;
@@ -619,7 +619,7 @@ GG_DEV int attempt_dp45_mixed(const DevParams& P, MixedRegs& S, const KS& K,
     // the 1080p Kerr frame 26.3 / 25.7 ms without / with the tenth root skipped)
     if (s2 < 8.0 || S.h <= P.min_step) {
       accepted = true;
-      const bool steady = S.h == P.max_step && s2 < 8.0 * kSteadyErr * kSteadyErr;
+      const bool steady = STEADY && S.h == P.max_step && s2 < 8.0 * kSteadyErr * kSteadyErr;
       if (s2 > 0.0 && !steady) {
         double hn = S.h * 0.9 * root10_8_over(s2);
         hn = hn < P.min_step ? P.min_step : (hn > P.max_step ? P.max_step : hn);

@@ -440,6 +440,19 @@ GG_API int gg_check_step_factor(const double* s2_dev, double* out_dev, uint64_t 
  * return conventions as above. */
 GG_API int gg_check_rcp(const float* x_dev, float* out_dev, uint64_t n, void* stream);
 
+/* Attempts of the trace kernels' steppers, one ray per sample of a width x
+ * height frame (at most 2^20 rays), from the camera until the ray ends or has
+ * made `attempts` of them (test use; no reference counterpart).  form 0: the
+ * reference's step, 1: full Dormand-Prince in FP64, 2: in mixed precision, up
+ * to its FP64 band.  steady 1: as the renders run, where an attempt at max_step
+ * whose errors are well inside their scales skips the step-size law; 0: every
+ * attempt takes the full law.  state_dev: n x 10 (x, v, lambda, next step);
+ * counts_dev: n x 3 (attempts, accepted, attempts at max_step). */
+GG_API int gg_check_steps(const gg_metric_t* metric, const gg_camera_t* camera,
+                          const gg_integrator_t* integ, uint32_t width, uint32_t height, int form,
+                          int steady, uint32_t attempts, double* state_dev, uint32_t* counts_dev,
+                          void* stream);
+
 /* The windows in which gg_backward takes an image back, on the host (test use;
  * no reference counterpart): counts[k] listed rays of n_keys - k segments each,
  * longest first, at most `most` segments a window (one ray at least).  Writes

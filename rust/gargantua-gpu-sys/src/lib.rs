@@ -249,6 +249,10 @@ extern "C" {
                                 stream: *mut c_void) -> c_int;
     pub fn gg_check_rcp(x_dev: *const f32, out_dev: *mut f32, n: u64,
                         stream: *mut c_void) -> c_int;
+    pub fn gg_check_steps(metric: *const gg_metric_t, camera: *const gg_camera_t,
+                          integ: *const gg_integrator_t, width: u32, height: u32, form: c_int,
+                          steady: c_int, attempts: u32, state_dev: *mut f64,
+                          counts_dev: *mut u32, stream: *mut c_void) -> c_int;
     pub fn gg_check_backward_windows(counts: *const u32, n_keys: u32, most: u64,
                                      windows: *mut u64, cap: u64, n: *mut u64) -> c_int;
     pub fn gg_check_backward_memory(ctx: *mut gg_ctx, memory: u64, largest: u64,
