@@ -176,6 +176,9 @@ _SIGNATURES = {
     "gg_check_steps": (C.c_int, [P(gg_metric_t), P(gg_camera_t), P(gg_integrator_t), C.c_uint32,
                                  C.c_uint32, C.c_int, C.c_int, C.c_uint32, C.c_void_p,
                                  C.c_void_p, C.c_void_p]),
+    "gg_check_trace_form": (C.c_int, [P(gg_metric_t), P(gg_camera_t), P(gg_disk_t),
+                                      P(gg_integrator_t), P(gg_render_opts_t), C.c_uint32,
+                                      C.c_uint32]),
     "gg_check_backward_windows": (C.c_int, [P(C.c_uint32), C.c_uint32, C.c_uint64,
                                             P(C.c_uint64), C.c_uint64, P(C.c_uint64)]),
     "gg_check_backward_memory": (C.c_int, [C.c_void_p, C.c_uint64, C.c_uint64, P(C.c_uint64),

@@ -265,3 +265,15 @@ extern "C" GG_API int gg_check_steps(const gg_metric_t* metric, const gg_camera_
                                                 counts_dev, s);
   return launch_status();
 }
+
+extern "C" GG_API int gg_check_trace_form(const gg_metric_t* metric, const gg_camera_t* camera,
+                                          const gg_disk_t* disk, const gg_integrator_t* integ,
+                                          const gg_render_opts_t* opts, uint32_t width,
+                                          uint32_t height) {
+  const int v = gg::validate_render(metric, camera, disk, integ, opts, width, height);
+  if (v != GG_OK) return v;
+  if (integ->precision != GG_PREC_FP64) return GG_ERR_UNSUPPORTED;
+  gg::DevParams P;
+  gg::make_params(metric, camera, disk, integ, opts, width, height, &P);
+  return gg::trace_form(P);
+}

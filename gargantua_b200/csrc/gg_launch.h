@@ -64,6 +64,10 @@ constexpr int kMixedMinBlocksReturned = GG_MIXED_RET_MIN_BLOCKS;
 constexpr int kMixedMinBlocksReturned = 4;
 #endif
 
+// The form of the trace kernel `P` selects: 0 the rolled one for many samples, 1
+// its smaller register budget's counterpart, 2 unrolled, 3 eight lanes a ray.
+int trace_form(const DevParams& P);
+
 // Resident CTAs per SM of the trace kernel `P` selects, and the CTAs that
 // give each of its rays a place at once.
 cudaError_t trace_occupancy(const DevParams& P, int* blocks_per_sm);

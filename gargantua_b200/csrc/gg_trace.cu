@@ -637,12 +637,20 @@ const void* select_group(const DevParams& P) {
 
 // Renders of so few samples are traced by the group kernel from the camera:
 // there each lane of the other kernels has at most one ray, and the time is one ray's
-// chain.  Lane per ray (unrolled) / group, ms: Schwarzschild with a thin disk at 64^2 0.93 /
-// 0.65, 100^2 1.12 / 0.81, 128^2 1.14 / 1.04, 165^2 1.39 / 1.54, 200^2 1.52 / 1.88; Kerr without
-// a disk 64^2 1.61 / 1.39, 128^2 1.79 / 1.96, 180^2 2.78 / 3.38.
-constexpr uint64_t kGroupRays = 1ull << 14;
+// chain.  The group kernel has 7,104 rays in flight, and its work per attempt is
+// larger, so the line lies a little above that; with the thin disk, whose rays
+// end early and unevenly, at twice as many.  Lane per ray (unrolled) / group, ms, at 64^2,
+// 90^2, 100^2, 128^2 (a view from 30 M, on the equator or, with the thin disk, at 80 deg):
+// Schwarzschild, no disk 0.85 / 0.76, 1.49 / 1.27, 1.09 / 1.23, 1.47 / 1.60; thin disk 0.85 / 0.65,
+// 1.06 / 0.80, 1.03 / 0.82, 1.04 / 1.00 (140^2: 1.10 / 1.14); volumetric disk 1.14 / 0.97, 1.92 / 1.60,
+// 1.38 / 1.60, 1.82 / 2.13; that with objects 1.45 / 1.20, 1.91 / 1.70, 1.73 / 1.97, 1.81 / 2.82.
+// Kerr, no disk 1.55 / 1.40, 3.77 / 3.45, 1.52 / 1.55, 1.68 / 2.05; thin disk 1.49 / 0.82, 1.48 / 1.05,
+// 1.40 / 1.10, 1.75 / 1.40 (160^2: 1.82 / 1.85); volumetric disk 2.06 / 1.78, 4.65 / 4.19, 2.02 / 2.18,
+// 2.13 / 2.85; that with objects 2.48 / 2.13, 5.58 / 5.03, 2.39 / 2.70, 2.60 / 3.80.
+constexpr uint64_t kGroupRays = 1ull << 13, kGroupRaysThin = 1ull << 14;
 bool group_render(const DevParams& P) {
-  return P.stepper == kStepperReference && !P.attempt_budget && P.n_rays <= kGroupRays;
+  return P.stepper == kStepperReference && !P.attempt_budget &&
+         P.n_rays <= (P.disk == kDiskThin ? kGroupRaysThin : kGroupRays);
 }
 
 // Kerr camera passes of fewer samples than this run the 4-CTA budget of the
@@ -664,18 +672,10 @@ const void* select_disk(const DevParams& P) {
   return trace_fn<METRIC, kDiskNone, STEPPER, kSrcCamera, false, false, false, SIZE>();
 }
 
-template <int STEPPER>
+template <int STEPPER, int SIZE>
 const void* select_metric(const DevParams& P) {
-  if (P.metric == kMetricKerr)
-    return P.n_rays < kSmallRender ? select_disk<kMetricKerr, STEPPER, kSizeSmall>(P)
-                                   : select_disk<kMetricKerr, STEPPER, kSizeLarge>(P);
-  return select_disk<kMetricSchwarzschild, STEPPER, kSizeLarge>(P);
-}
-
-template <int STEPPER>
-const void* select_chain(const DevParams& P) {
-  return P.metric == kMetricKerr ? select_disk<kMetricKerr, STEPPER, kSizeChain>(P)
-                                 : select_disk<kMetricSchwarzschild, STEPPER, kSizeChain>(P);
+  return P.metric == kMetricKerr ? select_disk<kMetricKerr, STEPPER, SIZE>(P)
+                                 : select_disk<kMetricSchwarzschild, STEPPER, SIZE>(P);
 }
 
 // Full Dormand-Prince camera passes of at most this many samples take the
@@ -689,20 +689,39 @@ constexpr uint64_t kChainRays = 3ull << 14;
 // 5.87; Kerr without a disk 200^2 3.66 / 3.37, 320^2 7.0 / 6.6, 500^2 10.99 / 11.00; with the
 // volumetric disk 200^2 4.72 / 4.39, 320^2 9.08 / 9.01, 450^2 14.2 / 15.4.
 constexpr uint64_t kChainRaysReference = 1ull << 18, kChainRaysVolumetric = 1ull << 17;
+
+uint64_t chain_rays(const DevParams& P) {
+  return P.stepper == kStepperDP45         ? kChainRays
+         : P.disk == kDiskVolumetric ? kChainRaysVolumetric
+                                     : kChainRaysReference;
+}
+
+// The form of the trace kernel that a render takes.
+enum TraceForm : int { kFormLarge, kFormSmall, kFormChain, kFormGroup };
+TraceForm form_of(const DevParams& P) {
+  if (group_render(P)) return kFormGroup;
+  if (P.n_rays <= chain_rays(P)) return kFormChain;
+  return P.metric == kMetricKerr && P.n_rays < kSmallRender ? kFormSmall : kFormLarge;
+}
+
+template <int STEPPER>
+const void* select_size(const DevParams& P, TraceForm form) {
+  if (form == kFormChain) return select_metric<STEPPER, kSizeChain>(P);
+  if (form == kFormSmall) return select_disk<kMetricKerr, STEPPER, kSizeSmall>(P);
+  return select_metric<STEPPER, kSizeLarge>(P);
+}
+
 const void* select_trace(const DevParams& P) {
-  if (group_render(P)) return select_group(P);
-  const bool full = P.stepper == kStepperDP45;
-  const bool chain = P.n_rays <= (full                        ? kChainRays
-                                  : P.disk == kDiskVolumetric ? kChainRaysVolumetric
-                                                              : kChainRaysReference);
+  const TraceForm form = form_of(P);
+  if (form == kFormGroup) return select_group(P);
   // gg_forward_ckpt admits only Kerr, the thin disk and the full stepper
   if (P.ckpt)
-    return chain ? trace_fn<kMetricKerr, kDiskThin, kStepperDP45, kSrcCamera, false, false, true,
-                            kSizeChain>()
-                 : trace_fn<kMetricKerr, kDiskThin, kStepperDP45, kSrcCamera, false, false, true>();
-  if (chain)
-    return full ? select_chain<kStepperDP45>(P) : select_chain<kStepperReference>(P);
-  return full ? select_metric<kStepperDP45>(P) : select_metric<kStepperReference>(P);
+    return form == kFormChain
+               ? trace_fn<kMetricKerr, kDiskThin, kStepperDP45, kSrcCamera, false, false, true,
+                          kSizeChain>()
+               : trace_fn<kMetricKerr, kDiskThin, kStepperDP45, kSrcCamera, false, false, true>();
+  return P.stepper == kStepperDP45 ? select_size<kStepperDP45>(P, form)
+                                   : select_size<kStepperReference>(P, form);
 }
 
 // The FP64 pass of the mixed form: full Dormand-Prince, thin disk or none.
@@ -733,6 +752,8 @@ cudaError_t trace_occupancy(const DevParams& P, int* blocks_per_sm) {
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, select_trace(P),
                                                        kTraceBlock, 0);
 }
+
+int trace_form(const DevParams& P) { return form_of(P); }
 
 int chain_capacity(const DevParams& P, int grid) {
   if (P.stepper != kStepperReference || P.attempt_budget || group_render(P)) return 0;

@@ -453,6 +453,14 @@ GG_API int gg_check_steps(const gg_metric_t* metric, const gg_camera_t* camera,
                           int steady, uint32_t attempts, double* state_dev, uint32_t* counts_dev,
                           void* stream);
 
+/* The form of the FP64 trace kernel that a render takes, on the host (test use;
+ * no reference counterpart): 0 or 1 a lane per ray with its stages in a loop (1:
+ * the budget of Kerr renders below 2^20 samples), 2 with its stages unrolled, 3 eight
+ * lanes per ray; a negative status if the render would be refused. */
+GG_API int gg_check_trace_form(const gg_metric_t* metric, const gg_camera_t* camera,
+                               const gg_disk_t* disk, const gg_integrator_t* integ,
+                               const gg_render_opts_t* opts, uint32_t width, uint32_t height);
+
 /* The windows in which gg_backward takes an image back, on the host (test use;
  * no reference counterpart): counts[k] listed rays of n_keys - k segments each,
  * longest first, at most `most` segments a window (one ray at least).  Writes

@@ -253,6 +253,9 @@ extern "C" {
                           integ: *const gg_integrator_t, width: u32, height: u32, form: c_int,
                           steady: c_int, attempts: u32, state_dev: *mut f64,
                           counts_dev: *mut u32, stream: *mut c_void) -> c_int;
+    pub fn gg_check_trace_form(metric: *const gg_metric_t, camera: *const gg_camera_t,
+                               disk: *const gg_disk_t, integ: *const gg_integrator_t,
+                               opts: *const gg_render_opts_t, width: u32, height: u32) -> c_int;
     pub fn gg_check_backward_windows(counts: *const u32, n_keys: u32, most: u64,
                                      windows: *mut u64, cap: u64, n: *mut u64) -> c_int;
     pub fn gg_check_backward_memory(ctx: *mut gg_ctx, memory: u64, largest: u64,
