@@ -362,39 +362,33 @@ class RayOutputs:
     """Host arrays of per-sample outcomes (``gg_ray_out_t``)."""
 
     def __init__(self, n: int):
-        self.n = n
-        self.cls = np.full(n, -1, np.int32)
-        self.x = np.zeros((4, n), np.float64)
-        self.v = np.zeros((4, n), np.float64)
-        self.lam = np.zeros(n, np.float64)
-        self.attempts = np.zeros(n, np.uint32)
-        self.accepted = np.zeros(n, np.uint32)
-        self.intensity = np.zeros(n, np.float64)
-        self.color_temp = np.zeros(n, np.float64)
-        self.rgb = np.zeros((n, 3), np.float64)
-        self.cross = np.zeros((8, n), np.float64)
+        self._allocate(n, np.zeros)
+        self.cls.fill(-1)
 
     @classmethod
     def _to_fill(cls, n: int) -> "RayOutputs":
         """The same arrays without initial values, for a render that writes
-        every entry, as parts of one block.  Filling 13 MB (256^2 samples)
-        first, in pages the system has to clear, took 1.2 ms of a 4.2 ms
-        call; and freed one by one, arrays of a few MB each went back to
-        the system and were mapped afresh by the next call (5.5 ms)."""
+        every entry.  Filling 13 MB (256^2 samples) first takes 0.9 ms of a
+        call of 4.0 ms.  As parts of one block they would stay mapped from one
+        call to the next when the results are dropped in turn (3.1 ms every time, where
+        these take 3.1 and 7.4 ms by turns, as the system takes their pages
+        back), but a caller who keeps one array would keep the block."""
         o = cls.__new__(cls)
-        o.n = n
-        parts = (("cls", (n,), np.int32), ("x", (4, n), np.float64), ("v", (4, n), np.float64),
-                 ("lam", (n,), np.float64), ("attempts", (n,), np.uint32),
-                 ("accepted", (n,), np.uint32), ("intensity", (n,), np.float64),
-                 ("color_temp", (n,), np.float64), ("rgb", (n, 3), np.float64),
-                 ("cross", (8, n), np.float64))
-        sizes = [int(np.prod(shape)) * np.dtype(kind).itemsize for _, shape, kind in parts]
-        block = np.empty(sum((size + 63) // 64 * 64 for size in sizes), np.uint8)
-        at = 0
-        for (name, shape, kind), size in zip(parts, sizes):
-            setattr(o, name, block[at:at + size].view(kind).reshape(shape))
-            at += (size + 63) // 64 * 64
+        o._allocate(n, np.empty)
         return o
+
+    def _allocate(self, n: int, new) -> None:
+        self.n = n
+        self.cls = new(n, np.int32)
+        self.x = new((4, n), np.float64)
+        self.v = new((4, n), np.float64)
+        self.lam = new(n, np.float64)
+        self.attempts = new(n, np.uint32)
+        self.accepted = new(n, np.uint32)
+        self.intensity = new(n, np.float64)
+        self.color_temp = new(n, np.float64)
+        self.rgb = new((n, 3), np.float64)
+        self.cross = new((8, n), np.float64)
 
     def struct(self) -> abi.gg_ray_out_t:
         def p(a, t):
