@@ -500,7 +500,8 @@ def run_ours(args) -> None:
                      "traffic_unit": "bytes per launch of trace_mixed_kernel",
                      "kernel": "trace_mixed_kernel<Kerr, ThinDisk> + FP64 band pass",
                      "flops_per_attempt": fpa,
-                     # the formulation the kernels run (closed-form sparse Christoffels)
+                     # the same attempt with the sparse Christoffels in closed form; the
+                     # kernels take fewer operations still (flops.py)
                      "flops_per_attempt_reduced": fpa_reduced,
                      "achieved_reduced": achieved * fpa_reduced / fpa / 1e12,
                      "frac_reduced": achieved * fpa_reduced / fpa / peak,

@@ -14,7 +14,7 @@
 // gg_trace.cu), which also stores each ray's state (x, v, next h) at the start
 // and after every kCkptEvery-th accepted step, and its DiffRay.
 //
-// Backward, over the disk rays with a nonzero dL/d(colour), in five launches:
+// Backward, over the disk rays with a nonzero dL/d(colour), in six launches:
 //   1. a counting sort lists the rays by their number of segments, longest
 //      first (backward_count / backward_scatter; the host makes the prefix
 //      sums in between);
@@ -43,10 +43,10 @@
 // The adjoint of t and phi is zero throughout (neither the metric nor the colour
 // depends on them), so six components are carried.  What bounds it: one ray's
 // chain.  Replayed and taken back by one lane, the longest ray of the 512^2
-// image (673 steps, the median being 39) took 8.6 ms, its warp issuing every
-// fourth cycle.  With the segments in parallel the longest chain is 32 to 128
-// steps, and the launches of the 512^2 backward take 0.9 (replay), 0.6 (crossing)
-// and 1.5 ms (chain): 9.2 ms before, 3.0 after; 128^2 2.95 / 0.72 ms.
+// image (673 steps, the median being 39) took the whole 8.6 ms, its warp issuing
+// every fourth cycle.  With the segments in parallel the longest chain is 32 to
+// 128 steps: 8.6 ms before, 3.0 after, 128^2 2.65 / 0.75 ms (CUDA events), of which
+// the 512^2 replay takes 0.9, the crossing 0.4 and the chain 1.7 ms.
 // The step sizes are held fixed (the adjoint of the discrete map with the
 // forward's accepted steps; their own dependence on the parameters moves the
 // solution by the truncation error only).

@@ -1031,51 +1031,51 @@ GG_DEV int attempt_dp45_fp64(const DevParams& P, Ray& R, const KS& K, bool& k1_v
     }
   } else {
 #pragma unroll 1
-  for (int s = s_first; s < 7; ++s) {
-    double px[4], pw[4], a[4];
-    // the last pass leaves the step's end in (px, pw)
-    auto step_end = [&]() {
+    for (int s = s_first; s < 7; ++s) {
+      double px[4], pw[4], a[4];
+      // the last pass leaves the step's end in (px, pw)
+      auto step_end = [&]() {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        xn[i] = px[i];
-        vn[i] = pw[i];
-      }
-      if (!(isfinite(px[0]) && isfinite(px[3]))) px[1] = -1.0;
-    };
-    if (CODE == kStageLooped) {
-      stage_state_looped(s, R, h, hh, K, px, pw);
-      if (s == 6) step_end();
-    } else {
-      switch (s) {
-        case 0:
+        for (int i = 0; i < 4; ++i) {
+          xn[i] = px[i];
+          vn[i] = pw[i];
+        }
+        if (!(isfinite(px[0]) && isfinite(px[3]))) px[1] = -1.0;
+      };
+      if (CODE == kStageLooped) {
+        stage_state_looped(s, R, h, hh, K, px, pw);
+        if (s == 6) step_end();
+      } else {
+        switch (s) {
+          case 0:
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            px[i] = R.x[i];
-            pw[i] = R.v[i];
-          }
-          break;
-        case 1: stage_state<1>(R, h, hh, K, px, pw); break;
-        case 2: stage_state<2>(R, h, hh, K, px, pw); break;
-        case 3: stage_state<3>(R, h, hh, K, px, pw); break;
-        case 4: stage_state<4>(R, h, hh, K, px, pw); break;
-        case 5: stage_state<5>(R, h, hh, K, px, pw); break;
-        default:
-          stage_state<6>(R, h, hh, K, px, pw);
-          step_end();
-          break;
+            for (int i = 0; i < 4; ++i) {
+              px[i] = R.x[i];
+              pw[i] = R.v[i];
+            }
+            break;
+          case 1: stage_state<1>(R, h, hh, K, px, pw); break;
+          case 2: stage_state<2>(R, h, hh, K, px, pw); break;
+          case 3: stage_state<3>(R, h, hh, K, px, pw); break;
+          case 4: stage_state<4>(R, h, hh, K, px, pw); break;
+          case 5: stage_state<5>(R, h, hh, K, px, pw); break;
+          default:
+            stage_state<6>(R, h, hh, K, px, pw);
+            step_end();
+            break;
+        }
       }
+      // is_valid_position; t and phi overflow only with a stage derivative that is not
+      // finite, which reaches r by the next stage, so they are tested at the last
+      if (s > 0 && !(isfinite(px[1]) && isfinite(px[2]) && px[1] > 0.0)) {
+        R.h = h * 0.5;
+        return kContinue;
+      }
+      Geometry<METRIC, kStepperDP45> G;
+      G.at(P, px[1], px[2]);
+      G.accel(pw, a);
+      K.set(s, a);
     }
-    // is_valid_position; t and phi overflow only with a stage derivative that is not
-    // finite, which reaches r by the next stage, so they are tested at the last
-    if (s > 0 && !(isfinite(px[1]) && isfinite(px[2]) && px[1] > 0.0)) {
-      R.h = h * 0.5;
-      return kContinue;
-    }
-    Geometry<METRIC, kStepperDP45> G;
-    G.at(P, px[1], px[2]);
-    G.accel(pw, a);
-    K.set(s, a);
-  }
   }
   // embedded error of positions (h^2 sum Ebar k) and velocities (h sum E k)
   double ex[4] = {0.0, 0.0, 0.0, 0.0}, ev[4] = {0.0, 0.0, 0.0, 0.0};

@@ -684,10 +684,15 @@ const void* select_metric(const DevParams& P) {
 // 2.65, 256^2 3.16 / 3.39, 512^2 7.2 / 8.5.
 constexpr uint64_t kChainRays = 3ull << 14;
 // The reference's step: up to 2^18, 2^17 with the volumetric disk, whose work at
-// every step wants more warps.  Rolled / unrolled, ms: Schwarzschild with a thin disk
-// at 200^2 1.90 / 1.52, 256^2 1.97 / 1.66, 400^2 3.16 / 2.69, 500^2 3.91 / 3.65, 700^2 5.75 /
-// 5.87; Kerr without a disk 200^2 3.66 / 3.37, 320^2 7.0 / 6.6, 500^2 10.99 / 11.00; with the
-// volumetric disk 200^2 4.72 / 4.39, 320^2 9.08 / 9.01, 450^2 14.2 / 15.4.
+// every step wants more warps.  One line for both metrics, where the slower one, Kerr,
+// has it.  Rolled / unrolled, ms: Kerr with a thin disk at 200^2 2.43 / 2.01, 400^2
+// 3.97 / 3.57, 512^2 4.29 / 4.22, 600^2 5.56 / 5.66, 700^2 6.9 / 7.4; volumetric disk 200^2 4.30 /
+// 3.86, 340^2 9.77 / 9.33, 362^2 11.9 / 11.8, 450^2 13.0 / 13.6; no disk 512^2 12.0 / 11.6;
+// Schwarzschild with a thin disk 512^2 3.43 / 2.91, 700^2 5.27 / 4.67, volumetric 362^2 5.16 /
+// 4.86, 600^2 9.3 / 9.5.  With objects the lines are within 5 % either way: Kerr 340^2 9.43 /
+// 9.46, 512^2 14.4 / 15.0, and the volumetric disk 256^2 11.6 / 11.9, 340^2 12.0 / 12.0, 362^2
+// 14.5 / 15.3; Schwarzschild 512^2 7.3 / 7.1, and the volumetric disk 340^2 5.73 / 5.44, 362^2
+// 6.86 / 6.92.
 constexpr uint64_t kChainRaysReference = 1ull << 18, kChainRaysVolumetric = 1ull << 17;
 
 uint64_t chain_rays(const DevParams& P) {

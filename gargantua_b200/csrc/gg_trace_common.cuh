@@ -46,9 +46,9 @@ constexpr int kMixedPeriod = GG_MIXED_PERIOD;
 constexpr uint32_t kChunk = 32;  // samples a warp takes from the queue at once
 // Attempts between refills of the group kernel, the lane of each group that
 // stands for it in a vote, and the rays a draining warp hands over.  A few
-// rays of an image take far more attempts than the rest (5,000 against 258 on
-// the Kerr view of the command line, whose rays near the axis make tiny
-// steps), and a warp left with them runs them at one or two lanes of 32.
+// near-critical rays of an image take far more attempts than the rest (up to
+// 5,000 against a median of 253 on the Kerr view of the command line), and a
+// warp left with them runs them at one or two lanes of 32.
 // Handing over at 0 (never) / 4 / 8 / 16 rays left, ms: Kerr sky 803x601 21.2 /
 // 15.7 / 15.7 / 15.7, lensed spheres with the disk 30.4 / 26.8 / 26.4 / 26.5,
 // Schwarzschild disk 800x600 13.3 / 12.9 / 12.8 / 12.8, the 1080p frame 35.1 /

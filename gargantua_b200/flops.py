@@ -29,10 +29,14 @@ DP45_ATTEMPT_FLOPS = {
 }
 
 
-# What the kernels compute instead: Kerr's right-hand side from its ~20
-# non-zero Christoffel symbols in closed form (one reciprocal, shared
-# subexpressions) rather than the dense 64-entry contraction, counted the
-# same way on the oracle's build with that arrangement (liboracle_gg_alt.so).
+# The same attempt with Kerr's right-hand side from its ~20 non-zero
+# Christoffel symbols in closed form (one reciprocal, shared subexpressions)
+# rather than the dense 64-entry contraction, counted the same way on the
+# oracle's build with that arrangement (liboracle_gg_alt.so).  The kernels
+# started from this form and do less: they halve the derivatives (about a dozen
+# operations fewer per right-hand side), take the constant products from the
+# host, and skip the error norm and the step law on most attempts.  So it is a
+# count of the method, not of the kernels' instructions, and no lower bound.
 # Schwarzschild's reference RHS is already the inlined sparse form.
 REDUCED_ATTEMPT_FLOPS = {
     (("kerr", "rtol"), 0): 1394,
@@ -48,7 +52,7 @@ def attempt_flops(metric_kind: str, rtol: float, stepper: int = 0) -> int:
 
 
 def reduced_attempt_flops(metric_kind: str, rtol: float, stepper: int = 0) -> int:
-    """FLOPs per attempt of the formulation the kernels run."""
+    """FLOPs per attempt with Kerr's right-hand side in closed form."""
     key = (metric_kind, "rtol" if rtol > 0.0 else "tol")
     if metric_kind != "kerr":
         return attempt_flops(metric_kind, rtol, stepper)
