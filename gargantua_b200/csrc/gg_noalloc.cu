@@ -76,6 +76,7 @@ extern "C" GG_API int gg_render_device_noalloc(const gg_metric_t* metric,
     return GG_ERR_UNSUPPORTED;
   gg::DevParams P;
   gg::make_params(metric, camera, disk, integ, opts, width, height, &P);
+  P.no_group_pass = 1;
   const bool want_image = rgb_dev != nullptr;
   const bool need_samples = want_image && P.spp > 1;
   if (need_samples && P.n_rays > kMaxSupersampled) return GG_ERR_TOO_LARGE;

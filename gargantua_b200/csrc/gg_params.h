@@ -99,7 +99,8 @@ struct DevParams {
   double sqrt_neg_gtt_obs;  // tracer.rs:93-94
   // disk
   int disk;
-  int pad1;
+  // gg_render_device_noalloc: no group pass follows, every ray ends in its lane
+  int no_group_pass;
   double r_inner, r_outer, scale_height, density_0, temperature_0, emissivity_index;
   double r_clear;  // volumetric: beyond this radius the disk's density is 0 everywhere
   // sky

@@ -647,10 +647,14 @@ const void* select_group(const DevParams& P) {
 // Kerr, no disk 1.55 / 1.40, 3.77 / 3.45, 1.52 / 1.55, 1.68 / 2.05; thin disk 1.49 / 0.82, 1.48 / 1.05,
 // 1.40 / 1.10, 1.75 / 1.40 (160^2: 1.82 / 1.85); volumetric disk 2.06 / 1.78, 4.65 / 4.19, 2.02 / 2.18,
 // 2.13 / 2.85; that with objects 2.48 / 2.13, 5.58 / 5.03, 2.39 / 2.70, 2.60 / 3.80.
-constexpr uint64_t kGroupRays = 1ull << 13, kGroupRaysThin = 1ull << 14;
+// Where no group pass follows a lane's last rays (gg_noalloc.cu), a near-critical ray
+// costs the other kernels twice as much, and the line stays at 2^14: 100^2, 110^2, 120^2,
+// Kerr without a disk 1.56 / 1.58, 5.5 / 4.1, 1.96 / 1.91.
+constexpr uint64_t kGroupRays = 1ull << 13, kGroupRaysFar = 1ull << 14;
 bool group_render(const DevParams& P) {
+  const bool far = P.disk == kDiskThin || P.no_group_pass;
   return P.stepper == kStepperReference && !P.attempt_budget &&
-         P.n_rays <= (P.disk == kDiskThin ? kGroupRaysThin : kGroupRays);
+         P.n_rays <= (far ? kGroupRaysFar : kGroupRays);
 }
 
 // Kerr camera passes of fewer samples than this run the 4-CTA budget of the
@@ -761,7 +765,8 @@ cudaError_t trace_occupancy(const DevParams& P, int* blocks_per_sm) {
 int trace_form(const DevParams& P) { return form_of(P); }
 
 int chain_capacity(const DevParams& P, int grid) {
-  if (P.stepper != kStepperReference || P.attempt_budget || group_render(P)) return 0;
+  if (P.stepper != kStepperReference || P.attempt_budget || P.no_group_pass || group_render(P))
+    return 0;
   return grid * (kTraceBlock / 32) * (int)kHandLanes;
 }
 
