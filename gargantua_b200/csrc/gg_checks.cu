@@ -249,7 +249,8 @@ extern "C" GG_API int gg_check_steps(const gg_metric_t* metric, const gg_camera_
                                      const gg_integrator_t* integ, uint32_t width,
                                      uint32_t height, int form, int steady, uint32_t attempts,
                                      double* state_dev, uint32_t* counts_dev, void* stream) {
-  if (!state_dev || !counts_dev || form < 0 || form > 2) return GG_ERR_INVALID_ARG;
+  if (!state_dev || !counts_dev || form < 0 || form > 2 || attempts > (1u << 16))
+    return GG_ERR_INVALID_ARG;
   gg_render_opts_t opts;
   gg_render_opts_default(&opts);
   const int v = gg::validate_render(metric, camera, nullptr, integ, &opts, width, height);

@@ -442,7 +442,7 @@ GG_API int gg_check_rcp(const float* x_dev, float* out_dev, uint64_t n, void* st
 
 /* Attempts of the trace kernels' steppers, one ray per sample of a width x
  * height frame (at most 2^20 rays), from the camera until the ray ends or has
- * made `attempts` of them (test use; no reference counterpart).  form 0: the
+ * made `attempts` of them (at most 2^16; test use; no reference counterpart).  form 0: the
  * reference's step, 1: full Dormand-Prince in FP64, 2: in mixed precision, up
  * to its FP64 band.  steady 1: as the renders run, where an attempt at max_step
  * whose errors are well inside their scales skips the step-size law; 0: every
