@@ -375,7 +375,8 @@ GG_DEV void mixed_stage(float r0, float th0, const MixedRegs& st, const KS& K, f
 // kerr_geometry in FP32 with the render's constant products (2M, a^2,
 // 2Ma, ... in DevParams) taken as given rather than rebuilt per evaluation,
 // and, as in KerrGeo64, halved derivatives whose factors 2 meet in the
-// contraction: the same symbols to the last bit (scalings by two are exact).
+// contraction: the same symbols to the last bit (scalings by two are exact),
+// but that an overflow sets in a factor 2 later.
 // Measured before / after: the 1080p Kerr frame 24.7 / 24.0 ms, the 64-scene
 // batch 85.0 / 83.9 ms.
 struct KerrGeo32 {

@@ -685,7 +685,9 @@ const void* select_metric(const DevParams& P) {
 // Full Dormand-Prince camera passes of at most this many samples take the
 // unrolled form.  Rolled / unrolled, ms, the differentiable forward: 64^2 1.83 /
 // 1.52, 128^2 2.84 / 2.32, 160^2 2.26 / 1.98, 200^2 2.53 / 2.34, 230^2 2.90 /
-// 2.65, 256^2 3.16 / 3.39, 512^2 7.2 / 8.5.
+// 2.65, 256^2 3.16 / 3.39, 512^2 7.2 / 8.5; with objects 200^2, Kerr 2.57 / 2.13,
+// Schwarzschild 1.88 / 1.45, and the volumetric disk 3.13 / 2.80 and 2.32 / 1.96, which
+// with objects turns at 260^2 (Kerr 4.95 / 4.57, Schwarzschild 2.68 / 2.93).
 constexpr uint64_t kChainRays = 3ull << 14;
 // The reference's step: up to 2^18, 2^17 with the volumetric disk, whose work at
 // every step wants more warps.  One line for both metrics, where the slower one, Kerr,

@@ -52,7 +52,9 @@ constexpr uint32_t kChunk = 32;  // samples a warp takes from the queue at once
 // Handing over at 0 (never) / 4 / 8 / 16 rays left, ms: Kerr sky 803x601 21.2 /
 // 15.7 / 15.7 / 15.7, lensed spheres with the disk 30.4 / 26.8 / 26.4 / 26.5,
 // Schwarzschild disk 800x600 13.3 / 12.9 / 12.8 / 12.8, the 1080p frame 35.1 /
-// 35.1 / 35.0 / 35.2.  Period 4 / 8 / 16: within the noise.
+// 35.1 / 35.0 / 35.2.  Thin-disk renders of 2^14 to 2^18 samples would do better
+// without (never / 8, Kerr 140^2 1.27 / 1.55, 256^2 2.15 / 2.65, 512^2 3.9 / 4.2).
+// Period 4 / 8 / 16: within the noise.
 #ifndef GG_GROUP_PERIOD
 #define GG_GROUP_PERIOD 8
 #endif
