@@ -330,10 +330,11 @@ void build_params(const gg_metric_t* metric, const gg_camera_t* camera, const gg
     const double m = P.mass, a = P.spin;
     P.a2_f = (float)(a * a);
     P.m2_f = (float)(2.0 * m);
-    P.ma_f = (float)(m * a);
+    P.mm2a2_f = (float)(-2.0 * a * a);
     P.m2a_f = (float)(2.0 * m * a);
-    P.ma2_f = (float)(m * a * a);
+    P.m4a_f = (float)(4.0 * m * a);
     P.m2a2_f = (float)(2.0 * m * a * a);
+    P.m4a2_f = (float)(4.0 * m * a * a);
     P.m2_d = 2.0 * m;
     P.a2_d = a * a;
     P.ma_d = m * a;

@@ -373,21 +373,10 @@ GG_DEV void mixed_stage(float r0, float th0, const MixedRegs& st, const KS& K, f
 }
 
 // kerr_geometry in FP32 with the render's constant products (2M, a^2,
-// 2Ma, ... in DevParams) taken as given rather than rebuilt per evaluation,
-// and, as in KerrGeo64, halved derivatives whose factors 2 meet in the
-// contraction: the same symbols to the last bit (scalings by two are exact),
-// but that an overflow sets in a factor 2 later.
-// Measured before / after: the 1080p Kerr frame 24.7 / 24.0 ms, the 64-scene
-// batch 85.0 / 83.9 ms.
-struct KerrGeo32 {
-  float h_tt_r, h_tt_th, h_rr_r, h_rr_th, h_thth_th, h_phph_r, h_phph_th, h_tph_r, h_tph_th;
-  float r;                   // dthth_r / 2
-  float gtt2, gtph2, gphph2;  // 2 g^tt, 2 g^tph, 2 g^phph
-  float n_rr, n_thth;         // g^rr, g^thth
-};
-
-GG_DEV KerrGeo32 kerr_geometry32(const DevParams& P, float r, float s, float c) {
-  KerrGeo32 G;
+// 2Ma, ... in DevParams) taken as given rather than rebuilt per evaluation:
+// the same symbols, a dozen fewer multiplies per right-hand side.
+GG_DEV KerrGeo<float> kerr_geometry32(const DevParams& P, float r, float s, float c) {
+  KerrGeo<float> G;
   const float a2 = P.a2_f;
   const float r2 = r * r, s2 = s * s, c2 = c * c, sc = s * c;
   const float sig = fmaf(a2, c2, r2);
@@ -403,23 +392,22 @@ GG_DEV KerrGeo32 kerr_geometry32(const DevParams& P, float r, float s, float c) 
   const float sm2r = fmaf(a2, c2, -r2);  // Sigma - 2 r^2
   const float sm2r_iS2 = sm2r * iS2;
   const float rsc_iS2 = r * (sc * iS2);
-  G.h_tt_r = P.mass_f * sm2r_iS2;
-  G.h_tt_th = P.m2a2_f * rsc_iS2;
-  G.h_rr_r = fmaf(a2, fmaf(r, s2, P.mass_f * c2), -P.mass_f * r2) * (iD * iD);
-  G.h_thth_th = -a2 * sc;
-  G.h_rr_th = G.h_thth_th * iD;
-  G.h_phph_r = fmaf(r, s2, P.ma2_f * (s2 * s2) * sm2r_iS2);
-  G.h_phph_th = fmaf(rho, sc, G.h_tt_th * s2 * (sig + rho));
-  G.h_tph_r = -P.ma_f * s2 * sm2r_iS2;
-  G.h_tph_th = -P.m2a_f * rsc_iS2 * rho;
+  G.dtt_r = P.m2_f * sm2r_iS2;
+  G.dtt_th = P.m4a2_f * rsc_iS2;
+  G.drr_r = 2.0f * fmaf(a2, fmaf(r, s2, P.mass_f * c2), -P.mass_f * r2) * (iD * iD);
+  G.drr_th = P.mm2a2_f * sc * iD;
+  G.dthth_r = 2.0f * r;
+  G.dthth_th = P.mm2a2_f * sc;
+  G.dphph_r = fmaf(2.0f * r, s2, P.m2a2_f * (s2 * s2) * sm2r_iS2);
+  G.dphph_th = fmaf(2.0f * rho, sc, P.m4a2_f * rsc_iS2 * s2 * (sig + rho));
+  G.dtph_r = -P.m2a_f * s2 * sm2r_iS2;
+  G.dtph_th = -P.m4a_f * rsc_iS2 * rho;
   const float big_a = fmaf(rho, rho, -a2 * del * s2);
-  const float iSD2 = iSD + iSD;
-  G.gtt2 = -big_a * iSD2;
-  G.gtph2 = -P.m2a_f * r * iSD2;
-  G.gphph2 = fmaf(-a2, s2, del) * iSD2 * is2;
-  G.n_rr = del * iS;
-  G.n_thth = iS;
-  G.r = r;
+  G.gtt = -big_a * iSD;
+  G.gtph = -P.m2a_f * r * iSD;
+  G.gphph = fmaf(-a2, s2, del) * iSD * is2;
+  G.hrr = -0.5f * del * iS;
+  G.hthth = -0.5f * iS;
   return G;
 }
 
@@ -427,28 +415,28 @@ GG_DEV KerrGeo32 kerr_geometry32(const DevParams& P, float r, float s, float c) 
 // sums: with A = G_tt vt + G_tph vph and B = G_tph vt + G_phph vph (per row),
 // G_tt vt^2 + 2 G_tph vt vph + G_phph vph^2 = vt A + vph B.  The same symbols,
 // four fewer operations per right-hand side.
-GG_DEV void kerr_contract32(const KerrGeo32& G, const float v[4], float acc[4]) {
+GG_DEV void kerr_contract32(const KerrGeo<float>& G, const float v[4], float acc[4]) {
   const float vt = v[0], vr = v[1], vth = v[2], vph = v[3];
-  const float Ar = fmaf(G.h_tph_r, vph, G.h_tt_r * vt);
-  const float Br = fmaf(G.h_phph_r, vph, G.h_tph_r * vt);
-  const float Ath = fmaf(G.h_tph_th, vph, G.h_tt_th * vt);
-  const float Bth = fmaf(G.h_phph_th, vph, G.h_tph_th * vt);
+  const float Ar = fmaf(G.dtph_r, vph, G.dtt_r * vt);
+  const float Br = fmaf(G.dphph_r, vph, G.dtph_r * vt);
+  const float Ath = fmaf(G.dtph_th, vph, G.dtt_th * vt);
+  const float Bth = fmaf(G.dphph_th, vph, G.dtph_th * vt);
   const float Et = fmaf(vth, Ath, vr * Ar);
   const float Ep = fmaf(vth, Bth, vr * Br);
-  acc[0] = -fmaf(G.gtph2, Ep, G.gtt2 * Et);
-  acc[3] = -fmaf(G.gphph2, Ep, G.gtph2 * Et);
+  acc[0] = -fmaf(G.gtph, Ep, G.gtt * Et);
+  acc[3] = -fmaf(G.gphph, Ep, G.gtph * Et);
   // r row: drr_r vr^2 + 2 drr_th vr vth - dthth_r vth^2 - (vt Ar + vph Br)
-  float w = vr * fmaf(G.h_rr_r, vr, (G.h_rr_th + G.h_rr_th) * vth);
-  w = fmaf(-G.r, vth * vth, w);
+  float w = vr * fmaf(G.drr_r, vr, (G.drr_th + G.drr_th) * vth);
+  w = fmaf(-G.dthth_r, vth * vth, w);
   w = fmaf(-vt, Ar, w);
   w = fmaf(-vph, Br, w);
-  acc[1] = -G.n_rr * w;
+  acc[1] = G.hrr * w;
   // theta row: dthth_th vth^2 + 2 dthth_r vr vth - drr_th vr^2 - (vt Ath + vph Bth)
-  float u = vth * fmaf(G.h_thth_th, vth, (G.r + G.r) * vr);
-  u = fmaf(-G.h_rr_th, vr * vr, u);
+  float u = vth * fmaf(G.dthth_th, vth, (G.dthth_r + G.dthth_r) * vr);
+  u = fmaf(-G.drr_th, vr * vr, u);
   u = fmaf(-vt, Ath, u);
   u = fmaf(-vph, Bth, u);
-  acc[2] = -G.n_thth * u;
+  acc[2] = G.hthth * u;
 }
 
 template <int METRIC>
@@ -456,7 +444,7 @@ struct Geometry32;
 
 template <>
 struct Geometry32<kMetricKerr> {
-  KerrGeo32 g;
+  KerrGeo<float> g;
   GG_DEV void at(const DevParams& P, float r, float th) {
     float s, c;
     sincos_polar(th, &s, &c);
