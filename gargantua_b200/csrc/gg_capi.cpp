@@ -337,8 +337,9 @@ void build_params(const gg_metric_t* metric, const gg_camera_t* camera, const gg
     P.m4a2_f = (float)(4.0 * m * a * a);
     P.m2_d = 2.0 * m;
     P.a2_d = a * a;
-    P.ma_d = m * a;
-    P.ma2_d = m * P.a2_d;
+    P.a2x2_d = 2.0 * P.a2_d;
+    P.m2a_d = 2.0 * (m * a);
+    P.m2a2_d = 2.0 * (m * P.a2_d);
   }
   P.max_radius_hi = (float)P.max_radius;
   P.max_radius_lo = (float)(P.max_radius - (double)P.max_radius_hi);

@@ -154,29 +154,30 @@ GG_DEV void schw_contract(const SchwGeoT<T>& G, const T v[4], T a[4]) {
   a[3] = T(-2) * G.ir * vr * vph - T(2) * G.g_ph_thph * vth * vph;
 }
 
-// The FP64 kernels' form of the Kerr pair above.  Every derivative there has a
-// factor 2 and both g^ii / 2 a factor 1/2: here the derivatives are halved
-// (h_*), and the factors that meet them carry the 2 (2 g^tt, 2 g^tph, 2 g^phph;
-// g^rr, g^thth).  Scaling by two is exact, so every rounding falls where
-// it fell before, and the render's constant products (2M, a^2, M a, M a^2,
-// DevParams) come from the host, rounded the same.  The sums are written with the fused
-// multiply-adds that nvcc forms for the pair above, so the result is that
-// pair's to the last bit in every kernel, whatever the compiler would fuse
-// there.  The kernels run against the FP64 pipe, two issue cycles an
-// instruction, and this form takes about a dozen fewer per evaluation.
-// Measured before / after: the 1080p Kerr frame 40.6 / 39.2 ms (drop-in) and
-// 50.8 / 48.5 ms (full Dormand-Prince), the 512^2 forward 8.11 / 7.79 ms.
+// The FP64 kernels' form of the Kerr pair above: the render's constant products
+// come from the host (DevParams), and the factors 2 and 4 sit in those and in
+// one 2 sin cos; scaling by two is exact, so every rounding falls where it fell
+// before.  The derivatives and -g^ii / 2 keep their size, so that the products with the
+// velocities also overflow where they did: inside the horizon velocities pass 1e150, and
+// halved derivatives gave such rays other infinities, and other attempts.  The sums are
+// written with the fused multiply-adds that nvcc forms for the pair above, so the
+// result is that pair's to the last bit in every kernel, whatever the compiler
+// would fuse there.  The kernels run against the FP64 pipe, two issue cycles an
+// instruction.
+// Measured where it took the plain pair's place, with halved derivatives: the 1080p Kerr
+// frame 40.6 / 39.2 ms (drop-in) and 50.8 / 48.5 ms (full Dormand-Prince), the 512^2
+// forward 8.11 / 7.79 ms; at their full size it takes 0.5 % more (35.2 / 35.4 and
+// 40.3 / 40.6 ms).
 struct KerrGeo64 {
-  double h_tt_r, h_tt_th, h_rr_r, h_rr_th, h_thth_th, h_phph_r, h_phph_th, h_tph_r, n_tph_th;
-  double r;                  // dthth_r / 2
-  double n_tt, n_tph, phph;  // -2 g^tt, -2 g^tph, 2 g^phph
-  double n_rr, n_thth;       // g^rr, g^thth
+  double dtt_r, dtt_th, drr_r, drr_th, dthth_r, dthth_th, dphph_r, dphph_th, dtph_r, n_tph_th;
+  double n_tt, n_tph, gphph;  // -g^tt, -g^tph, g^phph
+  double hrr, hthth;          // -g^rr / 2, -g^thth / 2
 };
 
 GG_DEV KerrGeo64 kerr_geometry64(const DevParams& P, double r, double s, double c) {
   KerrGeo64 G;
   const double a2 = P.a2_d;
-  const double r2 = r * r, s2 = s * s, c2 = c * c, sc = s * c;
+  const double r2 = r * r, s2 = s * s, c2 = c * c, sc = s * c, sc2 = sc + sc;
   const double ac = mul_rn(a2, c2);
   const double sig = add_rn(ac, r2);
   const double del = fma(r - P.m2_d, r, a2);
@@ -190,24 +191,23 @@ GG_DEV KerrGeo64 kerr_geometry64(const DevParams& P, double r, double s, double 
   const double iS2 = iS * iS;
   const double m2r = P.m2_d * r;
   const double sm2r = sub_rn(ac, r2);  // Sigma - 2 r^2
-  const double u = m2r * a2 * sc;
-  G.h_tt_r = P.mass * sm2r * iS2;
-  G.h_tt_th = u * iS2;
-  G.h_rr_r = fma(a2, fma(r, s2, mul_rn(P.mass, c2)), -mul_rn(P.mass, r2)) * (iD * iD);
-  G.h_thth_th = -a2 * sc;
-  G.h_rr_th = G.h_thth_th * iD;
-  G.h_phph_r = fma(r, s2, mul_rn(P.ma2_d * (s2 * s2) * sm2r, iS2));
-  G.h_phph_th = fma(rho, sc, mul_rn(u * s2 * add_rn(sig, rho), iS2));
-  G.h_tph_r = -P.ma_d * s2 * sm2r * iS2;
+  const double u = m2r * a2 * sc2;
+  G.dtt_r = P.m2_d * sm2r * iS2;
+  G.dtt_th = u * iS2;
+  G.drr_r = fma(P.a2x2_d, fma(r, s2, mul_rn(P.mass, c2)), -mul_rn(P.m2_d, r2)) * (iD * iD);
+  G.dthth_th = -a2 * sc2;
+  G.drr_th = G.dthth_th * iD;
+  G.dthth_r = r + r;
+  G.dphph_r = fma(G.dthth_r, s2, mul_rn(P.m2a2_d * (s2 * s2) * sm2r, iS2));
+  G.dphph_th = fma(rho, sc2, mul_rn(u * s2 * add_rn(sig, rho), iS2));
+  G.dtph_r = -P.m2a_d * s2 * sm2r * iS2;
   const double ma2r = m2r * P.spin;
-  G.n_tph_th = ma2r * sc * rho * iS2;
-  const double iSD2 = iSD + iSD;
-  G.n_tt = fma(rho, rho, -mul_rn(a2 * del, s2)) * iSD2;
-  G.n_tph = ma2r * iSD2;
-  G.phph = fma(-a2, s2, del) * iSD2 * is2;
-  G.n_rr = del * iS;
-  G.n_thth = iS;
-  G.r = r;
+  G.n_tph_th = ma2r * sc2 * rho * iS2;
+  G.n_tt = fma(rho, rho, -mul_rn(a2 * del, s2)) * iSD;
+  G.n_tph = ma2r * iSD;
+  G.gphph = fma(-a2, s2, del) * iSD * is2;
+  G.hthth = -0.5 * iS;
+  G.hrr = del * G.hthth;
   return G;
 }
 
@@ -216,28 +216,28 @@ GG_DEV KerrGeo64 kerr_geometry64(const DevParams& P, double r, double s, double 
 template <int STEPPER>
 GG_DEV void kerr_contract64(const KerrGeo64& G, const double v[4], double acc[4]) {
   const double vt = v[0], vr = v[1], vth = v[2], vph = v[3];
-  const double Et = fma(vr, fma(G.h_tt_r, vt, mul_rn(G.h_tph_r, vph)),
-                        mul_rn(vth, fma(G.h_tt_th, vt, -mul_rn(G.n_tph_th, vph))));
-  const double Ep = fma(vr, fma(G.h_tph_r, vt, mul_rn(G.h_phph_r, vph)),
-                        mul_rn(vth, fma(-G.n_tph_th, vt, mul_rn(G.h_phph_th, vph))));
+  const double Et = fma(vr, fma(G.dtt_r, vt, mul_rn(G.dtph_r, vph)),
+                        mul_rn(vth, fma(G.dtt_th, vt, -mul_rn(G.n_tph_th, vph))));
+  const double Ep = fma(vr, fma(G.dtph_r, vt, mul_rn(G.dphph_r, vph)),
+                        mul_rn(vth, fma(-G.n_tph_th, vt, mul_rn(G.dphph_th, vph))));
   acc[0] = STEPPER == kStepperDP45 ? fma(G.n_tph, Ep, mul_rn(G.n_tt, Et))
                                    : fma(G.n_tt, Et, mul_rn(G.n_tph, Ep));
-  acc[3] = fma(G.n_tph, Et, -mul_rn(G.phph, Ep));
+  acc[3] = fma(G.n_tph, Et, -mul_rn(G.gphph, Ep));
   const double vt2 = mul_rn(vt, vt), vr2 = mul_rn(vr, vr), vth2 = mul_rn(vth, vth),
                vph2 = mul_rn(vph, vph);
   const double two_tp = mul_rn(vt + vt, vph), two_rt = mul_rn(vr + vr, vth);
-  double x = fma(G.h_rr_r, vr2, -mul_rn(G.h_tt_r, vt2));
-  x = fma(-G.r, vth2, x);
-  x = fma(-G.h_phph_r, vph2, x);
-  x = fma(G.h_rr_th, two_rt, x);
-  x = fma(-G.h_tph_r, two_tp, x);
-  acc[1] = -G.n_rr * x;
-  double y = fma(G.h_thth_th, vth2, -mul_rn(G.h_tt_th, vt2));
-  y = fma(-G.h_rr_th, vr2, y);
-  y = fma(-G.h_phph_th, vph2, y);
-  y = fma(G.r, two_rt, y);
+  double x = fma(G.drr_r, vr2, -mul_rn(G.dtt_r, vt2));
+  x = fma(-G.dthth_r, vth2, x);
+  x = fma(-G.dphph_r, vph2, x);
+  x = fma(G.drr_th, two_rt, x);
+  x = fma(-G.dtph_r, two_tp, x);
+  acc[1] = G.hrr * x;
+  double y = fma(G.dthth_th, vth2, -mul_rn(G.dtt_th, vt2));
+  y = fma(-G.drr_th, vr2, y);
+  y = fma(-G.dphph_th, vph2, y);
+  y = fma(G.dthth_r, two_rt, y);
   y = fma(G.n_tph_th, two_tp, y);
-  acc[2] = -G.n_thth * y;
+  acc[2] = G.hthth * y;
 }
 
 // Schwarzschild likewise: the pair above with its halves and doubles taken out

@@ -79,8 +79,8 @@ struct DevParams {
   // the FP32 Kerr right-hand side's per-render constants: a^2, 2M, -2a^2,
   // 2Ma, 4Ma, 2Ma^2, 4Ma^2
   float a2_f, m2_f, mm2a2_f, m2a_f, m4a_f, m2a2_f, m4a2_f;
-  // the FP64 Kerr right-hand side's per-render constants: 2M, a^2, M a, M a^2
-  double m2_d, a2_d, ma_d, ma2_d;
+  // the FP64 Kerr right-hand side's per-render constants: 2M, a^2, 2a^2, 2Ma, 2Ma^2
+  double m2_d, a2_d, a2x2_d, m2a_d, m2a2_d;
   // sampling
   uint32_t width, height, spa, spp, jitter_spp, sub_w, sub_h;
   uint32_t pad0;
