@@ -70,7 +70,7 @@ UNIT = "geodesics/s"
 # (the second frame of a two-frame launch list, one pass, clocks not locked),
 # in the build with FP64 error sums.  They are the 6.2 MB image, the band
 # queue and the argument records of the once-per-ray finish and hand-off calls.
-MIXED_PASS_DRAM_BYTES = 3_209_984 + 37_537_280
+MIXED_PASS_DRAM_BYTES = 3_025_408 + 36_093_184
 # Renders of this many samples or more run the mixed form's hand-back rounds
 # (kHandBackMinRays in gargantua_b200/csrc/gg_capi.cpp).
 HAND_BACK_MIN_SAMPLES = 1 << 20

@@ -33,8 +33,7 @@ DP45_ATTEMPT_FLOPS = {
 # Christoffel symbols in closed form (one reciprocal, shared subexpressions)
 # rather than the dense 64-entry contraction, counted the same way on the
 # oracle's build with that arrangement (liboracle_gg_alt.so).  The kernels
-# started from this form and do less: they halve the derivatives (about a dozen
-# operations fewer per right-hand side), take the constant products from the
+# started from this form and do less: they take the constant products from the
 # host, and skip the error norm and the step law on most attempts.  So it is a
 # count of the method, not of the kernels' instructions, and no lower bound.
 # Schwarzschild's reference RHS is already the inlined sparse form.
